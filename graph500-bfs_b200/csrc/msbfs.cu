@@ -808,33 +808,169 @@ __global__ void fill_minus_one_kernel(int64_t* __restrict__ p, int64_t n) {
     p[i] = -1;
 }
 
-// pred of one root from its row levels: the entry row is its own parent,
-// every other reached row takes its first neighbour one level nearer.
-__global__ void batch_parent_kernel(const int32_t* __restrict__ lv, int64_t R,
-                                    const int64_t* __restrict__ row_ptr,
-                                    const int32_t* __restrict__ col,
-                                    const int32_t* __restrict__ inv, int root_row,
-                                    int64_t* __restrict__ pred, int* __restrict__ missing) {
-  for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < R;
-       v += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t L = lv[v];
-    if (L < 0) continue;
-    const int64_t me = inv[v];
-    if (v == root_row) {
-      pred[me] = pred_entry(me, L);
-      continue;
+// First of the neighbours col[jb, je) at level `want`, by the whole warp; -1
+// if there is none.  128 ids per step, so that four loads per lane are in
+// flight.
+__device__ __forceinline__ int32_t warp_find_level(const int32_t* __restrict__ lv,
+                                                   const int32_t* __restrict__ col, int64_t jb,
+                                                   int64_t je, int32_t want) {
+  const int lane = lane_id();
+  for (int64_t j = jb; j < je; j += 128) {
+    int32_t u[4], l[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int64_t x = j + q * 32 + lane;
+      u[q] = x < je ? __ldg(col + x) : -1;
     }
-    bool found = false;
-    for (int64_t j = row_ptr[v], e = row_ptr[v + 1]; j < e; ++j) {
-      const int32_t u = col[j];
-      if (lv[u] == L - 1) {
-        pred[me] = pred_entry(inv[u], L);
-        found = true;
-        break;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) l[q] = u[q] >= 0 ? __ldg(lv + u[q]) : -2;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const unsigned hit = __ballot_sync(kFull, l[q] == want);
+      if (hit) return __shfl_sync(kFull, u[q], __ffs(hit) - 1);
+    }
+  }
+  return -1;
+}
+
+constexpr int kParentProbe = 32;   // neighbours a lane tries before its warp sweeps the row
+constexpr int kParentPiece = 2048; // rows longer than this are left to batch_parent_piece_kernel
+
+// pred of one root from its row levels: the entry row is its own parent,
+// every other reached row takes a neighbour one level nearer (rows one level
+// below the entry row: the entry row itself).  A warp owns 32 rows.  Lists
+// are hub-first, so most rows end within a lane's few probes; the hub rows
+// themselves, whose only neighbours one level nearer may be a few low-degree
+// vertices at the end of millions of entries, are cut into pieces of
+// kParentPiece entries that a second kernel spreads over the grid.  What
+// bounds it is the longest serial scan: with a thread per row the hubs'
+// scans took 15-29 ms of a select at SCALE 24 and 0.9 ms at SCALE 18; now a
+// 33-root batch at SCALE 18 with every root selected and read back takes 4.0
+// instead of 33.6 ms, a 64-root batch at SCALE 24 with two roots 6.9 instead
+// of 38 ms.
+// pieces[0, cap): (row, piece) entries, count of them in *npieces; a row
+// that does not fit is swept here.
+__global__ void __launch_bounds__(256) batch_parent_kernel(
+    const int32_t* __restrict__ lv, int64_t R, const int64_t* __restrict__ row_ptr,
+    const int32_t* __restrict__ col, const int32_t* __restrict__ first,
+    const int32_t* __restrict__ inv, int root_row, int64_t* __restrict__ pred,
+    int2* __restrict__ pieces, int64_t cap, unsigned long long* __restrict__ npieces,
+    int* __restrict__ missing) {
+  const int lane = lane_id();
+  const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  const int64_t nchunks = (R + 31) >> 5;
+  const int32_t root_level = root_row >= 0 ? __ldg(lv + root_row) : -2;
+  for (int64_t ch = gw; ch < nchunks; ch += nwarps) {
+    const int64_t v = ch * 32 + lane;
+    const int32_t L = v < R ? __ldg(lv + v) : -1;
+    if (!__any_sync(kFull, L >= 0)) continue;
+    const bool open = L >= 0 && v != root_row;
+    int32_t par = -1;
+    int64_t j = 0, e = 0;
+    if (open) {
+      if (L == root_level + 1) {
+        par = root_row;
+      } else {
+        const int32_t f = __ldg(first + v);
+        if (__ldg(lv + f) == L - 1) {
+          par = f;
+        } else {
+          j = row_ptr[v] + 1;
+          e = row_ptr[v + 1];
+        }
       }
     }
-    if (!found) atomicExch(missing, 1);
+#pragma unroll 1
+    for (int p = 0; p < kParentProbe; p += 4) {
+      const bool need = par < 0 && j < e;
+      if (!__any_sync(kFull, need)) break;
+      if (need) {
+        const int64_t r = e - j;
+        int32_t u[4], l[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) u[q] = r > q ? __ldg(col + j + q) : -1;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) l[q] = u[q] >= 0 ? __ldg(lv + u[q]) : -2;
+#pragma unroll
+        for (int q = 3; q >= 0; --q)
+          if (l[q] == L - 1) par = u[q];
+        j += r < 4 ? r : 4;
+      }
+    }
+    unsigned rem = __ballot_sync(kFull, open && par < 0 && j < e);
+    bool deferred = false;
+    while (rem) {
+      const int l = __ffs(rem) - 1;
+      rem &= rem - 1;
+      const int64_t jb = __shfl_sync(kFull, j, l), je = __shfl_sync(kFull, e, l);
+      const int32_t want = __shfl_sync(kFull, L, l) - 1;
+      if (je - jb > kParentPiece) {
+        const int64_t n = (je - jb + kParentPiece - 1) / kParentPiece;
+        int64_t at = 0;
+        if (lane == 0) at = (int64_t)atomicAdd(npieces, (unsigned long long)n);
+        at = __shfl_sync(kFull, at, 0);
+        const bool fits = at + n <= cap;
+        // pieces reserved for a row that does not fit are marked empty
+        for (int64_t k = lane; k < n && at + k < cap; k += 32)
+          pieces[at + k] = make_int2(fits ? (int32_t)(ch * 32 + l) : -1, (int32_t)k);
+        if (fits) {
+          if (lane == l) deferred = true;
+          continue;
+        }
+      }
+      const int32_t p = warp_find_level(lv, col, jb, je, want);
+      if (lane == l) par = p;
+    }
+    if (open) {
+      if (par >= 0) pred[__ldg(inv + v)] = pred_entry(__ldg(inv + par), L);
+      else if (!deferred) atomicExch(missing, 1);
+    } else if (v == root_row && L >= 0) {
+      const int64_t me = __ldg(inv + v);
+      pred[me] = pred_entry(me, L);
+    }
   }
+}
+
+// The pieces batch_parent_kernel left: a warp scans one piece of a row's
+// last entries, unless another piece of the row has found a parent by then.
+// The pieces count from the end of the row, so that they do not depend on
+// how far its lane got (the first one may overlap what the lane tried).
+__global__ void __launch_bounds__(256) batch_parent_piece_kernel(
+    const int32_t* __restrict__ lv, const int64_t* __restrict__ row_ptr,
+    const int32_t* __restrict__ col, const int32_t* __restrict__ inv, int64_t* pred,
+    const int2* __restrict__ pieces, int64_t cap,
+    const unsigned long long* __restrict__ npieces) {
+  const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  const int64_t n = min((int64_t)*npieces, cap);
+  for (int64_t i = gw; i < n; i += nwarps) {
+    const int2 x = pieces[i];
+    if (x.x < 0) continue;
+    const int64_t me = __ldg(inv + x.x);
+    // one lane looks, so that the warp takes one branch
+    const int done = lane_id() == 0 ? __ldcg(pred + me) != -1 : 0;
+    if (__shfl_sync(kFull, done, 0)) continue;
+    const int64_t b = row_ptr[x.x], e = row_ptr[x.x + 1];
+    const int64_t je = e - (int64_t)x.y * kParentPiece;
+    const int64_t jb = max(b, je - kParentPiece);
+    const int32_t L = __ldg(lv + x.x);
+    const int32_t p = warp_find_level(lv, col, jb, je, L - 1);
+    if (p >= 0 && lane_id() == 0) pred[me] = pred_entry(__ldg(inv + p), L);
+  }
+}
+
+// Rows left to the pieces that none of them found a parent for.
+__global__ void batch_parent_check_kernel(const int32_t* __restrict__ inv,
+                                          const int64_t* __restrict__ pred,
+                                          const int2* __restrict__ pieces, int64_t cap,
+                                          const unsigned long long* __restrict__ npieces,
+                                          int* __restrict__ missing) {
+  const int64_t n = min((int64_t)*npieces, cap);
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x)
+    if (pieces[i].x >= 0 && pieces[i].y == 0 && pred[inv[pieces[i].x]] == -1)
+      atomicExch(missing, 1);
 }
 
 __global__ void set_entry_kernel(int64_t* p, int64_t i, int64_t value) { p[i] = value; }
@@ -1352,11 +1488,20 @@ void batch_select(const Graph& g, BfsState& st, const BatchState& bs, cudaStream
   batch_row_levels_kernel<<<grid_for(bs.R, B, sms, 8), B, 0, s>>>(bs.planes, bs.R, bs.levels,
                                                                  index, lv);
   fill_minus_one_kernel<<<grid_for(st.pred_size, B, sms, 8), B, 0, s>>>(st.pred, st.pred_size);
-  int* missing = reinterpret_cast<int*>(st.blk_cnt);  // scratch flag
-  check_cuda(cudaMemsetAsync(missing, 0, sizeof(int), s), "memset");
+  // scratch of the single-source search: a flag and a count in the block
+  // counts (two entries at least), the pieces of long rows in the degree prefix
+  int* missing = reinterpret_cast<int*>(st.blk_cnt);
+  unsigned long long* npieces = reinterpret_cast<unsigned long long*>(st.blk_cnt + 1);
+  int2* pieces = reinterpret_cast<int2*>(st.qdeg);
+  const int64_t cap = st.R + 2;
+  check_cuda(cudaMemsetAsync(st.blk_cnt, 0, 2 * sizeof(int64_t), s), "memset");
   const int root_row = bs.hctl->root_row[index];
-  batch_parent_kernel<<<grid_for(bs.R, B, sms, 8), B, 0, s>>>(lv, bs.R, c.row_ptr, c.col, c.inv,
-                                                              root_row, st.pred, missing);
+  batch_parent_kernel<<<grid_for(bs.R, B, sms, 8), B, 0, s>>>(
+      lv, bs.R, c.row_ptr, c.col, c.first, c.inv, root_row, st.pred, pieces, cap, npieces,
+      missing);
+  batch_parent_piece_kernel<<<sms * 8, B, 0, s>>>(lv, c.row_ptr, c.col, c.inv, st.pred, pieces,
+                                                  cap, npieces);
+  batch_parent_check_kernel<<<sms, B, 0, s>>>(c.inv, st.pred, pieces, cap, npieces, missing);
   const int64_t root = bs.roots[(size_t)index];
   if (g.core.enabled)
     core_write_tree(g, st.pred, bs.path_v[(size_t)index], bs.path_e[(size_t)index], s, sms);

@@ -221,3 +221,39 @@ def test_batch_root_levels_match_single_root(engine, scale, flags):
         assert np.array_equal(lv, single), (seed, lv, single)
         assert (lv <= 3).any() == (single <= 3).any()
     engine.end()
+
+
+@pytest.mark.parametrize("leaves", [3, 31, 33, 34, 2080, 2081, 2082, 4129, 20000])
+def test_batch_select_long_rows(engine, leaves):
+    """A hub whose only neighbour one level nearer the root is its last one:
+    root - x - hub - leaves on a ring, so that x (degree 2) comes after every
+    leaf (degree 3) in the hub's list; row lengths around the probe and piece
+    limits of the parent search."""
+    hub, x, root = leaves, leaves + 1, leaves + 2
+    i = np.arange(leaves)
+    edges = np.concatenate([np.stack([i, np.full(leaves, hub)], 1), np.stack([i, (i + 1) % leaves], 1),
+                            [[hub, x], [x, root]]]).astype(np.int64)
+    engine.build_from_edges(edges)
+    engine.prepare(16)
+    _check_batch(engine, edges, O.Graph(edges), [root, x, hub, 0])
+
+
+def test_batch_select_more_pieces_than_rows(engine):
+    """Bipartite and dense, with the root's neighbour last in every list of
+    the other side: more long rows to cut than the piece list has room for."""
+    na, nb = 2300, 6000
+    a, b = np.meshgrid(np.arange(na), na + np.arange(nb), indexing="ij")
+    keep = (a != 0) | (b < na + nb - 50)  # vertex 0 has the lowest degree of its side
+    root = na + nb
+    edges = np.concatenate([np.stack([a[keep], b[keep]], 1), [[0, root]]]).astype(np.int64)
+    engine.build_from_edges(edges)
+    engine.prepare(16)
+    engine.run_batch([root, 1], 16)
+    for k, r in enumerate((root, 1)):
+        engine.batch_select(k)
+        lv = engine.get_levels()
+        err, cnt = engine.validate(r)
+        assert err == 0 and cnt == len(edges)
+        engine.run(r)
+        assert np.array_equal(lv, engine.get_levels())
+        engine.run_batch([root, 1], 16)
