@@ -24,6 +24,7 @@
 #include <cstring>
 #include "common.cuh"
 #include "bfs_internal.h"
+#include "search_device.cuh"
 
 namespace b200bfs {
 namespace {
@@ -122,72 +123,12 @@ __global__ void reset_unvisited_kernel(const uint32_t* __restrict__ vis, int64_t
   }
 }
 
-// Assembly of pred from the row-order buffer rp (engine option
-// pred_assemble).  pmap[u] for original id u: its row (>= 0), -1 (no parent:
-// no edge, or beyond the graph), or -(p + 2) for a CoreBFS pruned vertex with
-// tree parent p.  A reached row gives its rp entry, an unreached row -1, a
-// pruned vertex its tree entry (level 0xFFFF, as write_tree_kernel writes),
-// the root itself.  The pass runs over u in order, so pred is written in full
-// lines; with group reordering the rows of a group of 2^16 ids are
-// contiguous, so the rp reads of the ids a wave of warps covers fall in a few
-// windows that stay in L2.  Scattering the entries by original id during the
-// levels instead costs a random 32-byte sector per entry.
-// A row's visited word and rp entry are loaded together (both only for
-// rows), so the entry costs one round trip after the map; nearly every row
-// is reached in a search of the giant component, so the rp reads of the
-// unreached rows are few.
-__device__ __forceinline__ int64_t assembled_entry(int32_t m, int64_t u,
-                                                   const uint32_t* __restrict__ vis,
-                                                   const int64_t* __restrict__ rp, int64_t root) {
-  int64_t e = -1;
-  if (m >= 0) {
-    const uint32_t vw = __ldg(vis + (m >> 5));
-    const int64_t r = __ldg(rp + m);
-    if ((vw >> (m & 31)) & 1u) e = r;
-  } else if (m < -1) {
-    e = pred_entry(-(int64_t)m - 2, 0xFFFF);
-  }
-  return u == root ? root : e;
-}
-
-// Four ids per thread: one 16-byte map load, two 16-byte pred stores
-// (pred and pmap are 256-byte aligned; n4 = n / 4, the tail done by thread 0).
-// sparse: pred already holds the entries of every vertex outside the
-// searched rows (-1, or its tree parent at level 0xFFFF), except at
-// prev_root (and the previous CoreBFS climb, which the caller restores), so
-// a group of four such vertices is not written: a third of the ids are rows
-// at SCALE 28, and one group in five has none.
-__device__ __forceinline__ void assemble_body(const int32_t* __restrict__ pmap, int64_t n,
-                                              const uint32_t* __restrict__ vis,
-                                              const int64_t* __restrict__ rp, int64_t root,
-                                              int64_t prev_root, int sparse,
-                                              int64_t* __restrict__ pred) {
-  const int64_t n4 = n >> 2;
-  const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  const int4* m4 = reinterpret_cast<const int4*>(pmap);
-  longlong2* p2 = reinterpret_cast<longlong2*>(pred);
-  for (int64_t i = t0; i < n4; i += stride) {
-    const int4 m = __ldg(m4 + i);
-    const int64_t u = 4 * i;
-    if (sparse && (m.x & m.y & m.z & m.w) < 0 && (uint64_t)(root - u) >= 4 &&
-        (uint64_t)(prev_root - u) >= 4)
-      continue;
-    p2[2 * i] = make_longlong2(assembled_entry(m.x, u, vis, rp, root),
-                               assembled_entry(m.y, u + 1, vis, rp, root));
-    p2[2 * i + 1] = make_longlong2(assembled_entry(m.z, u + 2, vis, rp, root),
-                                   assembled_entry(m.w, u + 3, vis, rp, root));
-  }
-  if (t0 == 0)
-    for (int64_t u = 4 * n4; u < n; ++u) pred[u] = assembled_entry(pmap[u], u, vis, rp, root);
-}
-
 __global__ void assemble_pred_kernel(const int32_t* __restrict__ pmap, int64_t n,
                                      const uint32_t* __restrict__ vis,
                                      const int64_t* __restrict__ rp, int64_t root,
                                      int64_t prev_root, int sparse,
                                      int64_t* __restrict__ pred) {
-  assemble_body(pmap, n, vis, rp, root, prev_root, sparse, pred);
+  assemble_body<false>(pmap, n, vis, rp, root, prev_root, sparse, pred);
 }
 
 // Number of 4-id groups of pmap (n4 of them) holding a searched row.
@@ -427,173 +368,6 @@ __global__ void __launch_bounds__(256) bu_kernel(const uint32_t* __restrict__ cu
   publish_if_last(ctr, pub, seq);
 }
 
-// Bottom-up step, second form: a warp step covers kWords bitmap words, so
-// every lane owns kWords vertices and issues their row-offset loads, then
-// their neighbour-id loads (two neighbours per round), then the visited
-// probes, back to back: kWords * 2 independent loads are in flight per lane
-// instead of one dependent chain.  Rows unresolved after 8 probes are swept
-// by the whole warp as in bu_kernel.
-// kFirst: each open row first probes its first neighbour, read from the
-// dense fpair[] array together with that neighbour's original id (one
-// coalesced 8-byte read per row), and loads its row offsets only when that
-// probe misses; the offset rounds then start at the second neighbour.  A
-// parent found by the first probe has its pred entry's id at hand: no
-// second load, no gather into inv[].
-// kSpec (with kFirst): the fpair[] loads are issued for every row of the
-// words, beside the loads of the words themselves, and the visited rows'
-// entries are dropped afterwards: one round trip fewer per step, for the
-// levels where most rows are still unvisited.
-// The row search of the bottom-up forms for kWords bitmap words w[k] (w[k]
-// < 0: no word) whose current visited words are c[k]: lane l handles row
-// w[k] * 32 + l of each word, and the word's next value c[k] | found is
-// written to nxt.
-template <int kWords, bool kFirst, bool kSpec = false>
-__device__ __forceinline__ void bu_rows(
-    const int64_t (&w)[kWords], const uint32_t (&c)[kWords], const uint32_t* __restrict__ cur,
-    uint32_t* __restrict__ nxt, const int64_t* __restrict__ row_ptr,
-    const int32_t* __restrict__ col, const int2* __restrict__ fpair,
-    const int32_t* __restrict__ inv, const int32_t* __restrict__ pidx,
-    int64_t* __restrict__ pred, int64_t level, uint32_t& found_total, uint32_t& scanned) {
-  const int lane = lane_id();
-  // open row w[k] * 32 + lane: its next neighbour is col[b[k]] and
-  // rem[k] of them are left (a row has fewer than 2^31 neighbours)
-  int64_t b[kWords];
-  int32_t rem[kWords];
-  // par[k]: the parent's row id, or with pf[k] (found by the first probe)
-  // already its original id
-  int32_t par[kWords];
-  bool pf[kWords];
-  if (kFirst) {
-    int2 f[kWords];
-#pragma unroll
-    for (int k = 0; k < kWords; ++k) {
-      par[k] = -1;
-      pf[k] = false;
-      b[k] = 0;
-      rem[k] = 0;
-      f[k] = make_int2(-1, -1);
-      if (kSpec ? w[k] >= 0 : (((~c[k]) >> lane) & 1u) != 0)
-        f[k] = __ldg(fpair + w[k] * 32 + lane);
-    }
-    if (kSpec) {
-#pragma unroll
-      for (int k = 0; k < kWords; ++k)
-        if (((c[k] >> lane) & 1u) != 0) f[k].x = -1;
-    }
-    uint32_t mf[kWords];
-#pragma unroll
-    for (int k = 0; k < kWords; ++k) mf[k] = f[k].x >= 0 ? __ldg(cur + (f[k].x >> 5)) : 0u;
-#pragma unroll
-    for (int k = 0; k < kWords; ++k) {
-      if (f[k].x < 0) continue;
-      scanned += 1;
-      if ((mf[k] >> (f[k].x & 31)) & 1u) {
-        par[k] = f[k].y;
-        pf[k] = true;
-      } else {
-        const int64_t v = w[k] * 32 + lane;
-        const int64_t rb = row_ptr[v];
-        b[k] = rb + 1;
-        rem[k] = (int32_t)(row_ptr[v + 1] - rb - 1);
-      }
-    }
-  } else {
-#pragma unroll
-    for (int k = 0; k < kWords; ++k) {
-      par[k] = -1;
-      pf[k] = false;
-      b[k] = 0;
-      rem[k] = 0;
-      if (((~c[k]) >> lane) & 1u) {
-        const int64_t v = w[k] * 32 + lane;
-        b[k] = row_ptr[v];
-        rem[k] = (int32_t)(row_ptr[v + 1] - b[k]);
-      }
-    }
-  }
-  // four rounds of two probes per vertex
-#pragma unroll
-  for (int round = 0; round < 4; ++round) {
-    int32_t u0[kWords], u1[kWords];
-    bool need = false;
-#pragma unroll
-    for (int k = 0; k < kWords; ++k) {
-      u0[k] = u1[k] = -1;
-      if (par[k] < 0 && rem[k] > 0) {
-        u0[k] = __ldg(col + b[k]);
-        if (rem[k] > 1) u1[k] = __ldg(col + b[k] + 1);
-        need = true;
-      }
-    }
-    if (!__any_sync(kFull, need)) break;
-    uint32_t m0[kWords], m1[kWords];
-#pragma unroll
-    for (int k = 0; k < kWords; ++k) {
-      m0[k] = u0[k] >= 0 ? __ldg(cur + (u0[k] >> 5)) : 0u;
-      m1[k] = u1[k] >= 0 ? __ldg(cur + (u1[k] >> 5)) : 0u;
-    }
-#pragma unroll
-    for (int k = 0; k < kWords; ++k) {
-      if (u0[k] < 0) continue;
-      if ((m0[k] >> (u0[k] & 31)) & 1u) {
-        par[k] = u0[k];
-        scanned += 1;
-      } else if (u1[k] >= 0 && ((m1[k] >> (u1[k] & 31)) & 1u)) {
-        par[k] = u1[k];
-        scanned += 2;
-      } else {
-        const int32_t t = (u1[k] >= 0) ? 2 : 1;
-        scanned += t;
-        b[k] += t;
-        rem[k] -= t;
-      }
-    }
-  }
-  // cooperative sweep of the rows still unresolved
-#pragma unroll
-  for (int k = 0; k < kWords; ++k) {
-    unsigned left = __ballot_sync(kFull, par[k] < 0 && rem[k] > 0);
-    while (left) {
-      const int l = __ffs(left) - 1;
-      left &= left - 1;
-      const int64_t jb = __shfl_sync(kFull, b[k], l);
-      const int64_t je = jb + __shfl_sync(kFull, rem[k], l);
-      int32_t p = -1;
-      for (int64_t j = jb; j < je; j += 32) {
-        const int64_t jj = j + lane;
-        int32_t u = 0;
-        bool hit = false;
-        if (jj < je) {
-          u = __ldg(col + jj);
-          hit = bit_test(cur, u);
-        }
-        const unsigned hm = __ballot_sync(kFull, hit);
-        if (hm) {
-          const int fl = __ffs(hm) - 1;
-          p = __shfl_sync(kFull, u, fl);
-          if (lane == l) scanned += (uint32_t)(j - jb + fl + 1);
-          break;
-        }
-      }
-      if (p < 0 && lane == l) scanned += (uint32_t)(je - jb);
-      if (lane == l) par[k] = p;
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < kWords; ++k) {
-    const unsigned fm = __ballot_sync(kFull, par[k] >= 0);
-    if (lane == 0 && w[k] >= 0) {
-      nxt[w[k]] = c[k] | fm;
-      found_total += __popc(fm);
-    }
-    if (par[k] >= 0) {
-      const int64_t v = w[k] * 32 + lane;
-      const int32_t po = pf[k] ? par[k] : __ldg(inv + par[k]);
-      pred[pred_slot(pidx, v)] = pred_entry(po, level);
-    }
-  }
-}
-
 template <int kWords, bool kFirst, bool kSparse, bool kSpec = false>
 __device__ __forceinline__ void bu_wide_body(
     const uint32_t* __restrict__ cur, uint32_t* __restrict__ nxt, int64_t W,
@@ -601,67 +375,14 @@ __device__ __forceinline__ void bu_wide_body(
     const int2* __restrict__ fpair, const int32_t* __restrict__ inv,
     const int32_t* __restrict__ pidx, int64_t* __restrict__ pred, int64_t level,
     Counters* __restrict__ ctr) {
-  const int lane = lane_id();
-  const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  // per-lane counts (a lane scans far fewer than 2^32 entries), added to
-  // the 64-bit level counters once at the end
+  // per-lane counts, added to the 64-bit level counters once at the end
   uint32_t found_total = 0, scanned = 0;
-  if (kSparse) {
-    // Few unvisited rows left (the last levels): a warp takes blocks of 32
-    // bitmap words, one per lane; full words are copied to nxt at once and
-    // only the words with unvisited rows go through the row search, kWords
-    // at a time.  A block costs one load per lane instead of 32 / kWords
-    // dependent word steps.
-    const int64_t nblk = (W + 31) >> 5;
-    for (int64_t blk = gw; blk < nblk; blk += nwarps) {
-      const int64_t wl = (blk << 5) + lane;
-      const uint32_t cl = wl < W ? cur[wl] : kFull;
-      if (cl == kFull && wl < W) nxt[wl] = kFull;
-      unsigned om = __ballot_sync(kFull, cl != kFull);
-      while (om) {
-        int64_t w[kWords];
-        uint32_t c[kWords];
-#pragma unroll
-        for (int k = 0; k < kWords; ++k) {
-          w[k] = -1;
-          c[k] = kFull;
-          if (om) {
-            const int l = __ffs(om) - 1;
-            om &= om - 1;
-            w[k] = (blk << 5) + l;
-            c[k] = __shfl_sync(kFull, cl, l);
-          }
-        }
-        bu_rows<kWords, kFirst>(w, c, cur, nxt, row_ptr, col, fpair, inv, pidx, pred,
-                                level, found_total, scanned);
-      }
-    }
-  } else {
-    // kWords consecutive words per warp step, strided over the warps
-    for (int64_t w0 = gw * kWords; w0 < W; w0 += nwarps * kWords) {
-      int64_t w[kWords];
-      uint32_t c[kWords];
-      bool all_full = true;
-#pragma unroll
-      for (int k = 0; k < kWords; ++k) {
-        w[k] = w0 + k < W ? w0 + k : -1;
-        c[k] = w[k] >= 0 ? cur[w0 + k] : kFull;
-        all_full &= (c[k] == kFull);
-      }
-      // (kSpec issues the row loads before the words arrive: no early exit)
-      if (!kSpec && all_full) {
-        if (lane < kWords && w0 + lane < W) nxt[w0 + lane] = kFull;
-        continue;
-      }
-      bu_rows<kWords, kFirst, kSpec>(w, c, cur, nxt, row_ptr, col, fpair, inv, pidx, pred, level,
-                              found_total, scanned);
-    }
-  }
+  bu_wide_words<kWords, kFirst, kSparse, kSpec>(cur, nxt, W, row_ptr, col, fpair, inv, pidx, pred,
+                                                level, found_total, scanned);
   unsigned long long sc = scanned;
 #pragma unroll
   for (int o = 16; o; o >>= 1) sc += __shfl_xor_sync(kFull, sc, o);
-  if (lane == 0) {
+  if (lane_id() == 0) {
     if (found_total) atomicAdd(&ctr->nq, (unsigned long long)found_total);
     if (sc) atomicAdd(&ctr->scanned, sc);
   }
@@ -1295,7 +1016,7 @@ __global__ void sg_assemble_kernel(const SingleCtl* __restrict__ c, const SgArg*
                                    uint32_t* const* __restrict__ vis_pp,
                                    const int32_t* __restrict__ pmap, int64_t n,
                                    const int64_t* __restrict__ rp, int64_t* __restrict__ pred) {
-  assemble_body(pmap, n, vis_pp[c->cur], rp, a->root, a->sparse ? a->prev_root : -1, a->sparse,
+  assemble_body<false>(pmap, n, vis_pp[c->cur], rp, a->root, a->sparse ? a->prev_root : -1, a->sparse,
                 pred);
 }
 
@@ -1527,6 +1248,14 @@ void BfsState::allocate(DeviceArena& arena, const Graph& g) {
   check_cuda(cudaHostGetDevicePointer(&dpub, hpub, 0), "mapped counters");
   hpub->seq = 0;
   pub_seq = 0;
+  pctl = arena_alloc<PersistCtl>(arena, 1, "search kernel control block");
+  queue2 = arena_alloc<int32_t>(arena, R + 1, "frontier queue");
+  prec = arena_alloc<PersistRec>(arena, kMaxLevel, "level records");
+  check_cuda(cudaMemset(pctl, 0, sizeof(PersistCtl)), "search kernel control block");
+  check_cuda(cudaHostAlloc(&hout, sizeof(PersistOut), cudaHostAllocMapped), "mapped result");
+  check_cuda(cudaHostGetDevicePointer(&dout, hout, 0), "mapped result");
+  hout->seq = 0;
+  out_seq = 0;
   sctl = arena_alloc<SingleCtl>(arena, 1, "search control block");
   sarg = arena_alloc<SgArg>(arena, 1, "search arguments");
   d_vis = arena_alloc<uint32_t*>(arena, 2, "bitmap pointers");
@@ -1580,6 +1309,14 @@ void BfsState::release(DeviceArena& arena) {
   if (pmap) arena.free(pmap);
   rp = nullptr;
   pmap = nullptr;
+  arena.free(pctl);
+  arena.free(queue2);
+  queue2 = nullptr;
+  arena.free(prec);
+  if (hout) cudaFreeHost(hout);
+  pctl = nullptr;
+  prec = nullptr;
+  hout = dout = nullptr;
   if (hpub) cudaFreeHost(hpub);
   hpub = nullptr;
   dpub = nullptr;
@@ -1800,6 +1537,9 @@ static Counters wait_level(BfsState& st, cudaStream_t s) {
 void run_bfs_core(const Graph& g, BfsState& st, cudaStream_t s, int sms, int64_t root,
                   int64_t root_level, int edgefactor, double alpha, double beta, int64_t* at,
                   const RunOptions& opt, b200bfs_run_stats* stats) {
+  if (use_persistent(g, opt) && run_bfs_core_persistent(g, st, s, sms, root, root_level,
+                                                        edgefactor, alpha, beta, at, opt, stats))
+    return;
   // the device-driven loop has top-down forms 1, 3, 4 and 5 and its own
   // bottom-up form (four words per warp step, as form 4)
   if (opt.single_graph && opt.td_kernel != 2 && opt.td_kernel <= 5) {
@@ -2036,6 +1776,8 @@ void run_bfs_core(const Graph& g, BfsState& st, cudaStream_t s, int sms, int64_t
   st.prev_root = root;
   st.assembled = assemble;
   check_cuda(cudaGetLastError(), "bfs");
+  // the last level published its counters before its event was reached
+  check_cuda(cudaEventSynchronize(st.ev[timed.back().second + 1]), "last level");
   for (size_t k = 0; k < timed.size(); ++k) {
     const auto& t = timed[k];
     float ms = 0;

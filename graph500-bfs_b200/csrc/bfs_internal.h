@@ -43,6 +43,51 @@ struct SingleCtl {
   SgRec rec[kSgHist];
 };
 
+// The search as one kernel (persistent.cu).
+struct PersistCounters {         // of one level
+  unsigned long long q;          // next frontier's list: rows << 32 | their adjacency entries
+  unsigned long long nq;         // vertices discovered that are not in the list
+  unsigned long long nq_edges;   // pre-dedup degree sum of all discovered (top-down)
+  unsigned long long scanned;    // adjacency entries read bottom-up
+};
+struct PersistCtl {              // zero between searches
+  unsigned bar, blocks_done, error, pad;
+  unsigned long long stamp;      // when the assembly began
+  PersistCounters c[3];          // of level L: c[L % 3]
+};
+struct PersistRec {
+  int32_t level, bottom_up;
+  long long input, discovered, scanned, ns;
+};
+constexpr int kPersistRecs = 64;  // level records published with the result
+struct PersistOut {              // host-mapped
+  long long level, visited, pred_ns, at[9];
+  int nrec, done;                // done: 1 finished, 3 too many levels, 4 gave up
+  unsigned at_set, pad;          // slots of at that were written
+  PersistRec rec[kPersistRecs];
+  unsigned long long seq;        // written last
+};
+struct PersistArgs {
+  const int64_t* row_ptr;
+  const int32_t *col, *inv, *mdeg, *rank;
+  const int2* fpair;
+  int64_t R, W, nedges;
+  uint32_t* vis[2];
+  int32_t* rows[2];              // frontier lists: rows and
+  uint32_t* pre[2];              // their degree prefix
+  int64_t* rp;
+  const int32_t* pmap;
+  int64_t* pred;
+  int64_t pred_size;
+  PersistCtl* ctl;
+  PersistOut* out;
+  PersistRec* more;              // records past kPersistRecs
+  int64_t root, prev_root, root_level;
+  double alpha, beta;
+  int edgefactor, force_direction, sparse, pad;
+  unsigned long long seq;
+};
+
 struct BfsState {
   bool allocated = false;
   int64_t R = 0, W = 0, pred_size = 0, nblk = 0;
@@ -87,6 +132,13 @@ struct BfsState {
   // their entries from the search before); core_groups counts those groups
   bool asm_sparse = false;
   int64_t core_groups = 0;
+  // search as one kernel
+  PersistCtl* pctl = nullptr;
+  int32_t* queue2 = nullptr;              // second frontier list
+  PersistRec* prec = nullptr;             // [kMaxLevel] records past kPersistRecs
+  PersistOut* hout = nullptr;             // result, host-mapped (dout: device address)
+  PersistOut* dout = nullptr;
+  unsigned long long out_seq = 0;
   // device-driven level loop (graph mode)
   SingleCtl* sctl = nullptr;
   SingleCtl* hsctl = nullptr;             // pinned mirror
@@ -140,6 +192,10 @@ struct RunOptions {
   // forms only: bottom-up form 4, top-down forms 1, 3, 4, 5); 0: host loop
   // with per-level kernel timings
   int single_graph = 0;
+  // The search as one kernel (persistent.cu).  0: never (the level loop);
+  // 1: by the rule of use_persistent; 2 and 3: on every graph it can take,
+  // with 1024 or 2048 threads per SM.
+  int persistent = 1;
   double batch_alpha = 30;  // batched search: alpha used when the caller passes alpha <= 0
 };
 
@@ -147,9 +203,33 @@ void run_bfs_core(const Graph& g, BfsState& st, cudaStream_t s, int sms, int64_t
                   int64_t root_level, int edgefactor, double alpha, double beta, int64_t* at,
                   const RunOptions& opt, b200bfs_run_stats* stats);
 
+// The search as one cooperative kernel (persistent.cu); same results and
+// statistics as run_bfs_core.  Needs the pred assembly.  False: nothing was
+// launched, because its blocks cannot all be resident.
+bool run_bfs_core_persistent(const Graph& g, BfsState& st, cudaStream_t s, int sms, int64_t root,
+                             int64_t root_level, int edgefactor, double alpha, double beta,
+                             int64_t* at, const RunOptions& opt, b200bfs_run_stats* stats);
+
 void levels_from_pred(const BfsState& st, cudaStream_t s, int sms, int32_t* d_levels);
 
 inline bool use_pred_assembly(const Graph&, const RunOptions& o) { return o.pred_assemble != 0; }
+// Whether a search goes to the one kernel.  It has its own level code, so
+// options that pick a form of the level loop keep the level loop.  Its
+// frontier lists keep degree prefixes in 32 bits.  Its top-down levels count
+// the vertices they claim by their returning OR, where the level loop counts
+// them in a pass over the bitmaps: dearer on the levels that claim tens of
+// millions of vertices, which from SCALE 27 on outweighs the launches saved
+// (us per search, level loop / one kernel: SCALE 26 973 / 856, SCALE 27
+// 2243 / 2488 plain and 1567 / 1567 with CoreBFS; 33 M and 63 M rows).
+inline bool use_persistent(const Graph& g, const RunOptions& o) {
+  if (o.persistent == 0 || !use_pred_assembly(g, o) || o.single_graph) return false;
+  if (g.csr.nedges >= int64_t(1) << 32 || !g.csr.first_pair) return false;
+  if (o.persistent > 1) return true;
+  const RunOptions d;
+  return g.csr.nrows < int64_t(3) << 24 && o.bu_kernel == d.bu_kernel &&
+         o.td_kernel == d.td_kernel && o.bu_probe == d.bu_probe && o.bu_first == d.bu_first &&
+         o.bu_sparse == d.bu_sparse && o.bu_spec == d.bu_spec && o.td_unroll == d.td_unroll;
+}
 // Allocates rp and pmap (if needed) and fills pmap from the current row map
 // and tree parents; synchronises the stream.
 void build_pred_assembly(DeviceArena& arena, const Graph& g, BfsState& st, cudaStream_t s,

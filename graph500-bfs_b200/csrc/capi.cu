@@ -560,6 +560,9 @@ int b200bfs_set_option(b200bfs_handle* h, const char* name, int64_t value) {
     } else if (n == "force_direction") {
       require(value >= 0 && value <= 2, B200BFS_ERR_INVALID, "force_direction must be 0..2");
       e.opt.force_direction = (int)value;
+    } else if (n == "persistent") {
+      require(value >= 0 && value <= 3, B200BFS_ERR_INVALID, "persistent must be 0..3");
+      e.opt.persistent = (int)value;
     } else if (n == "batch_probe") {
       require(value == 4 || value == 8 || value == 16 || value == 32 || value == 64 ||
                   value == 128 || value == 256 || value == 1024,
