@@ -943,12 +943,35 @@ __global__ void __launch_bounds__(kFrontierThreads) frontier_write_kernel(
   frontier_write_body(fr, W, row_ptr, blk_cnt, blk_deg, queue, qdeg);
 }
 
+// Level of a vertex from its pred entry.  A CoreBFS tree vertex off the climb
+// carries the unknown level 0xFFFF: its level is that of the first vertex up
+// its parent chain with a known one, plus the steps (a chain has at most as
+// many as there were pruning rounds, 32); -1 if the chain is not reached.
+__device__ __forceinline__ int32_t level_of_entry(int64_t e, const int64_t* __restrict__ pred) {
+  if (e == -1) return -1;
+  int32_t d = (int32_t)(((uint64_t)e >> 48) & 0xFFFF);
+  for (int32_t up = 1; d == 0xFFFF && up <= 64; ++up) {
+    e = __ldg(pred + (e & 0xFFFFFFFFFFFFll));
+    if (e == -1) return -1;
+    const int32_t x = (int32_t)(((uint64_t)e >> 48) & 0xFFFF);
+    if (x != 0xFFFF) return x + up;
+  }
+  return d;
+}
+
+// Four ids per thread (n is a multiple of 4; both arrays are 256-byte
+// aligned): one pass over pred and one over the levels is all that is left of
+// it (SCALE 26 with CoreBFS: 127 us, and 379 us in five further passes over
+// the tree vertices, before).
 __global__ void levels_kernel(const int64_t* __restrict__ pred, int64_t n,
                               int32_t* __restrict__ lv) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+  const longlong2* p2 = reinterpret_cast<const longlong2*>(pred);
+  int4* l4 = reinterpret_cast<int4*>(lv);
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n / 4;
        i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t p = pred[i];
-    lv[i] = (p == -1) ? -1 : (int32_t)(((uint64_t)p >> 48) & 0xFFFF);
+    const longlong2 a = __ldg(p2 + 2 * i), b = __ldg(p2 + 2 * i + 1);
+    l4[i] = make_int4(level_of_entry(a.x, pred), level_of_entry(a.y, pred),
+                      level_of_entry(b.x, pred), level_of_entry(b.y, pred));
   }
 }
 
@@ -1229,7 +1252,7 @@ void build_pred_assembly(DeviceArena& arena, const Graph& g, BfsState& st, cudaS
   st.core_groups = (int64_t)h;
 }
 
-void BfsState::allocate(DeviceArena& arena, const Graph& g) {
+void BfsState::allocate(DeviceArena& arena, const Graph& g, cudaStream_t s) {
   release(arena);
   R = g.csr.nrows;
   W = (R + 31) / 32;
@@ -1244,27 +1267,39 @@ void BfsState::allocate(DeviceArena& arena, const Graph& g) {
   blk_deg = arena_alloc<int64_t>(arena, nblk + 1, "block degrees");
   pred = arena_alloc<int64_t>(arena, pred_size + 2, "pred");
   ctr = arena_alloc<Counters>(arena, 1, "counters");
-  check_cuda(cudaHostAlloc(&hpub, sizeof(Published), cudaHostAllocMapped), "mapped counters");
-  check_cuda(cudaHostGetDevicePointer(&dpub, hpub, 0), "mapped counters");
-  hpub->seq = 0;
+  // one pinned, mapped block for everything the host and the device exchange
+  struct HostBlock {
+    Published pub;
+    PersistOut out;
+    SingleCtl sctl;
+    SgArg sarg;
+  };
+  HostBlock *hb = nullptr, *db = nullptr;
+  check_cuda(cudaHostAlloc(&hblock, sizeof(HostBlock), cudaHostAllocMapped), "mapped memory");
+  hb = static_cast<HostBlock*>(hblock);
+  check_cuda(cudaHostGetDevicePointer(&db, hblock, 0), "mapped memory");
+  memset(hblock, 0, sizeof(HostBlock));
+  hpub = &hb->pub;
+  dpub = &db->pub;
+  hout = &hb->out;
+  dout = &db->out;
+  hsctl = &hb->sctl;
+  hsarg = &hb->sarg;
   pub_seq = 0;
+  out_seq = 0;
   pctl = arena_alloc<PersistCtl>(arena, 1, "search kernel control block");
   queue2 = arena_alloc<int32_t>(arena, R + 1, "frontier queue");
-  prec = arena_alloc<PersistRec>(arena, kMaxLevel, "level records");
-  check_cuda(cudaMemset(pctl, 0, sizeof(PersistCtl)), "search kernel control block");
-  check_cuda(cudaHostAlloc(&hout, sizeof(PersistOut), cudaHostAllocMapped), "mapped result");
-  check_cuda(cudaHostGetDevicePointer(&dout, hout, 0), "mapped result");
-  hout->seq = 0;
-  out_seq = 0;
+  prec = arena_alloc<PersistRec>(arena, std::min<int64_t>(kMaxLevel, R + 1), "level records");
+  check_cuda(cudaMemsetAsync(pctl, 0, sizeof(PersistCtl), s), "search kernel control block");
   sctl = arena_alloc<SingleCtl>(arena, 1, "search control block");
   sarg = arena_alloc<SgArg>(arena, 1, "search arguments");
   d_vis = arena_alloc<uint32_t*>(arena, 2, "bitmap pointers");
   pred_clean = false;
   prev_root = -1;
   assembled = false;
-  check_cuda(cudaMemcpy(d_vis, vis, sizeof(vis), cudaMemcpyHostToDevice), "bitmap pointers");
-  check_cuda(cudaMallocHost(&hsctl, sizeof(SingleCtl)), "pinned control block");
-  check_cuda(cudaMallocHost(&hsarg, sizeof(SgArg)), "pinned arguments");
+  check_cuda(cudaMemcpyAsync(d_vis, vis, sizeof(vis), cudaMemcpyHostToDevice, s),
+             "bitmap pointers");
+  check_cuda(cudaStreamSynchronize(s), "search buffers");
   allocated = true;
 }
 
@@ -1290,8 +1325,6 @@ void BfsState::release(DeviceArena& arena) {
   arena.free(sarg);
   arena.free(d_vis);
   d_vis = nullptr;
-  cudaFreeHost(hsctl);
-  cudaFreeHost(hsarg);
   sctl = nullptr;
   sarg = nullptr;
   hsctl = nullptr;
@@ -1313,11 +1346,11 @@ void BfsState::release(DeviceArena& arena) {
   arena.free(queue2);
   queue2 = nullptr;
   arena.free(prec);
-  if (hout) cudaFreeHost(hout);
   pctl = nullptr;
   prec = nullptr;
   hout = dout = nullptr;
-  if (hpub) cudaFreeHost(hpub);
+  if (hblock) cudaFreeHost(hblock);
+  hblock = nullptr;
   hpub = nullptr;
   dpub = nullptr;
   allocated = false;
@@ -1802,7 +1835,7 @@ void finish_run_stats(BfsState& st, b200bfs_run_stats* stats) {
 }
 
 void levels_from_pred(const BfsState& st, cudaStream_t s, int sms, int32_t* d_levels) {
-  levels_kernel<<<grid_for(st.pred_size, 256, sms, 8), 256, 0, s>>>(st.pred, st.pred_size,
+  levels_kernel<<<grid_for(st.pred_size / 4, 256, sms, 8), 256, 0, s>>>(st.pred, st.pred_size,
                                                                    d_levels);
 }
 

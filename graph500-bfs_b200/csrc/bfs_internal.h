@@ -55,9 +55,8 @@ struct PersistCtl {              // zero between searches
   unsigned long long stamp;      // when the assembly began
   PersistCounters c[3];          // of level L: c[L % 3]
 };
-struct PersistRec {
-  int32_t level, bottom_up;
-  long long input, discovered, scanned, ns;
+struct PersistRec {              // of one level; the graph has less than 2^32 entries
+  uint32_t bottom_up, discovered, scanned, ns;
 };
 constexpr int kPersistRecs = 64;  // level records published with the result
 struct PersistOut {              // host-mapped
@@ -135,13 +134,14 @@ struct BfsState {
   // search as one kernel
   PersistCtl* pctl = nullptr;
   int32_t* queue2 = nullptr;              // second frontier list
-  PersistRec* prec = nullptr;             // [kMaxLevel] records past kPersistRecs
+  PersistRec* prec = nullptr;             // level records past kPersistRecs (R + 1 at most)
   PersistOut* hout = nullptr;             // result, host-mapped (dout: device address)
   PersistOut* dout = nullptr;
   unsigned long long out_seq = 0;
   // device-driven level loop (graph mode)
   SingleCtl* sctl = nullptr;
   SingleCtl* hsctl = nullptr;             // pinned mirror
+  void* hblock = nullptr;                 // the pinned memory of hpub, hout, hsctl and hsarg
   SgArg* sarg = nullptr;
   uint32_t** d_vis = nullptr;             // device copy of vis[2]
   SgArg* hsarg = nullptr;                 // pinned staging
@@ -151,7 +151,7 @@ struct BfsState {
 
   cudaEvent_t event(size_t i);            // creates events on demand
 
-  void allocate(DeviceArena& arena, const Graph& g);
+  void allocate(DeviceArena& arena, const Graph& g, cudaStream_t s);
   void release(DeviceArena& arena);
 };
 

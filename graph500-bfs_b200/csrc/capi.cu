@@ -35,8 +35,31 @@ void* DeviceArena::alloc(size_t bytes, const char* what) {
       throw Error{B200BFS_ERR_OOM, std::string("shared HBM budget exceeded allocating ") + what};
     }
   }
+  // a kept block that is at most an eighth too large (small ones: up to twice)
+  const size_t most = bytes < (size_t(1) << 20) ? 2 * bytes : bytes + bytes / 8;
+  size_t best = kept_.size();
+  for (size_t i = 0; i < kept_.size(); ++i)
+    if (kept_[i].size >= bytes && kept_[i].size <= most &&
+        (best == kept_.size() || kept_[i].size < kept_[best].size))
+      best = i;
+  if (best < kept_.size()) {
+    const Block b = kept_[best];
+    kept_[best] = kept_.back();
+    kept_.pop_back();
+    kept_bytes_ -= b.size;
+    in_use_ += bytes;
+    live_.push_back({b.p, bytes, b.size, seq_++});
+    return b.p;
+  }
   void* p = nullptr;
   cudaError_t e = cudaMalloc(&p, bytes);
+  if (e == cudaErrorMemoryAllocation && !kept_.empty()) {
+    cudaGetLastError();
+    for (const Block& b : kept_) cudaFree(b.p);
+    kept_.clear();
+    kept_bytes_ = 0;
+    e = cudaMalloc(&p, bytes);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     if (shared_) shared_->used.fetch_sub(bytes);
@@ -44,8 +67,32 @@ void* DeviceArena::alloc(size_t bytes, const char* what) {
                                      std::to_string(bytes) + " bytes)"};
   }
   in_use_ += bytes;
-  live_.push_back({p, bytes, seq_++});
+  live_.push_back({p, bytes, bytes, seq_++});
   return p;
+}
+
+void DeviceArena::give(const Block& b) {
+  in_use_ -= b.bytes;
+  if (shared_) shared_->used.fetch_sub(b.bytes);
+  if (keep_ && b.size <= limit_ && kept_bytes_ <= limit_ - b.size) {
+    kept_.push_back(b);
+    kept_bytes_ += b.size;
+  } else {
+    cudaFree(b.p);
+  }
+}
+
+// Keeps the smallest blocks (the costliest per byte).
+void DeviceArena::settle(uint64_t spare) {
+  std::lock_guard<std::mutex> lock(mu_);
+  limit_ = spare;
+  std::sort(kept_.begin(), kept_.end(),
+            [](const Block& a, const Block& b) { return a.size < b.size; });
+  while (kept_bytes_ > limit_) {
+    cudaFree(kept_.back().p);
+    kept_bytes_ -= kept_.back().size;
+    kept_.pop_back();
+  }
 }
 
 void DeviceArena::free(void* p) {
@@ -53,11 +100,10 @@ void DeviceArena::free(void* p) {
   std::lock_guard<std::mutex> lock(mu_);
   for (size_t i = 0; i < live_.size(); ++i)
     if (live_[i].p == p) {
-      in_use_ -= live_[i].bytes;
-      if (shared_) shared_->used.fetch_sub(live_[i].bytes);
+      const Block b = live_[i];
       live_[i] = live_.back();
       live_.pop_back();
-      cudaFree(p);
+      give(b);
       return;
     }
 }
@@ -66,11 +112,10 @@ void DeviceArena::rollback(uint64_t m) {
   std::lock_guard<std::mutex> lock(mu_);
   for (size_t i = 0; i < live_.size();) {
     if (live_[i].seq >= m) {
-      in_use_ -= live_[i].bytes;
-      if (shared_) shared_->used.fetch_sub(live_[i].bytes);
-      cudaFree(live_[i].p);
+      const Block b = live_[i];
       live_[i] = live_.back();
       live_.pop_back();
+      give(b);
     } else {
       ++i;
     }
@@ -159,6 +204,7 @@ int b200bfs_create(const b200bfs_config* cfg, b200bfs_handle** out) {
     b200bfs::check_cuda(cudaStreamCreateWithFlags(&e.stream, cudaStreamNonBlocking), "stream");
     b200bfs::check_cuda(cudaEventCreate(&e.run_ev[0]), "event");
     b200bfs::check_cuda(cudaEventCreate(&e.run_ev[1]), "event");
+    e.arena.open();
   });
   if (rc != B200BFS_OK) {
     delete h;
@@ -172,6 +218,7 @@ int b200bfs_destroy(b200bfs_handle* h) {
   if (!h) return B200BFS_ERR_INVALID;
   guarded(h, [&](Engine& e) {
     e.free_graph();
+    e.arena.settle(0);
     for (cudaEvent_t& ev : e.run_ev)
       if (ev) cudaEventDestroy(ev);
     if (e.stream) cudaStreamDestroy(e.stream);
@@ -402,7 +449,7 @@ int b200bfs_prepare(b200bfs_handle* h, int edgefactor, double alpha, double beta
     require(e.g.built, B200BFS_ERR_STATE, "no graph built");
     require(alpha > 0 && beta > 0 && edgefactor > 0, B200BFS_ERR_INVALID, "bad parameters");
     e.prepared = false;
-    e.st.allocate(e.arena, e.g);
+    e.st.allocate(e.arena, e.g, e.stream);
     try {
       if (e.g.core.enabled) {
         // reads reachability from pred as the level kernels leave it
@@ -418,6 +465,7 @@ int b200bfs_prepare(b200bfs_handle* h, int edgefactor, double alpha, double beta
       e.st.release(e.arena);
       throw;
     }
+    e.settle_memory();
     e.prepared = true;
   });
 }
@@ -514,7 +562,6 @@ int b200bfs_get_levels(b200bfs_handle* h, int32_t* levels) {
     require(e.have_run, B200BFS_ERR_STATE, "no search has run");
     int32_t* d = b200bfs::arena_alloc<int32_t>(e.arena, e.g.pred_size, "levels");
     b200bfs::levels_from_pred(e.st, e.stream, e.sms, d);
-    if (e.g.core.enabled) b200bfs::core_fill_levels(e.g, e.st, e.stream, e.sms, d);
     b200bfs::check_cuda(
         cudaMemcpyAsync(levels, d, e.g.pred_size * 4, cudaMemcpyDeviceToHost, e.stream), "copy");
     b200bfs::check_cuda(cudaStreamSynchronize(e.stream), "get_levels");
@@ -574,8 +621,10 @@ int b200bfs_set_option(b200bfs_handle* h, const char* name, int64_t value) {
     } else if (n == "pred_assemble") {
       require(value == 0 || value == 1, B200BFS_ERR_INVALID, "pred_assemble must be 0 or 1");
       e.opt.pred_assemble = (int)value;
-      if (e.prepared && !e.st.pmap && b200bfs::use_pred_assembly(e.g, e.opt))
+      if (e.prepared && !e.st.pmap && b200bfs::use_pred_assembly(e.g, e.opt)) {
         b200bfs::build_pred_assembly(e.arena, e.g, e.st, e.stream, e.sms);
+        e.settle_memory();
+      }
     } else {
       throw b200bfs::Error{B200BFS_ERR_INVALID, "unknown option " + n};
     }
@@ -610,6 +659,7 @@ int b200bfs_end(b200bfs_handle* h) {
   return guarded(h, [&](Engine& e) {
     if (e.st.allocated) e.st.release(e.arena);
     e.bs.release(e.arena);
+    e.arena.settle(0);
     e.prepared = false;
     e.have_run = false;
   });
@@ -625,9 +675,11 @@ int b200bfs_run_batch(b200bfs_handle* h, const int64_t* roots, int num_roots, in
     for (int i = 0; i < num_roots; ++i)
       require(roots[i] >= 0 && roots[i] < e.g.nverts, B200BFS_ERR_INVALID, "root out of range");
     b200bfs_batch_stats rs;
+    const uint64_t held = e.arena.in_use();
     b200bfs::ensure_batch_view(e.arena, e.g, e.stream, e.sms);
     b200bfs::run_batch(e.arena, e.g, e.bs, e.stream, e.sms, roots, num_roots, edgefactor,
                        alpha > 0 ? alpha : e.opt.batch_alpha, beta, e.opt.batch_graph != 0, &rs);
+    if (e.arena.in_use() != held) e.settle_memory();  // a first batch, or more planes
     e.st.levels = e.bs.level_records;
     if (stats) *stats = rs;
     e.have_run = false;

@@ -240,18 +240,6 @@ __global__ void write_path_kernel(PathArg p, int64_t* __restrict__ pred) {
   for (int i = threadIdx.x; i < p.n; i += blockDim.x) pred[p.v[i]] = p.e[i];
 }
 
-__global__ void fill_levels_kernel(const int2* __restrict__ list, int64_t n,
-                                   int32_t* __restrict__ lv) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const int2 t = list[i];
-    if (lv[t.x] != 0xFFFF) continue;
-    const int32_t lp = lv[t.y];
-    if (lp == -1) lv[t.x] = -1;
-    else if (lp != 0xFFFF) lv[t.x] = lp + 1;
-  }
-}
-
 __global__ void has_edge_kernel(const int32_t* __restrict__ rank,
                                 const int32_t* __restrict__ tp, int64_t n, int64_t pred_size,
                                 uint8_t* __restrict__ out) {
@@ -539,14 +527,6 @@ void core_run_bfs(const Graph& g, BfsState& st, cudaStream_t s, int sms, int64_t
     stats->algorithmic_bytes += bytes;
     stats->kernel_launches += launches;
   }
-}
-
-void core_fill_levels(const Graph& g, const BfsState& st, cudaStream_t s, int sms,
-                      int32_t* d_levels) {
-  const int64_t nt = g.core.tree_vertices;
-  if (nt == 0) return;
-  for (int pass = 0; pass <= g.core.rounds + 1; ++pass)
-    fill_levels_kernel<<<grid_for(nt, 256, sms, 8), 256, 0, s>>>(g.core.tree_list, nt, d_levels);
 }
 
 void has_edge_all(const Graph& g, cudaStream_t s, int sms, uint8_t* d_out) {

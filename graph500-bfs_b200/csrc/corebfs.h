@@ -24,10 +24,6 @@ void core_climb(const Graph& g, int64_t root, std::vector<int64_t>& path_v,
 // tree parent with level 0xFFFF, then the climbed path.  Returns launches.
 int core_write_tree(const Graph& g, int64_t* pred, const std::vector<int64_t>& path_v,
                     const std::vector<int64_t>& path_e, cudaStream_t s, int sms);
-// Exact levels of pruned vertices from their parents (d_levels holds the
-// levels taken from pred, 0xFFFF for pruned vertices).
-void core_fill_levels(const Graph& g, const BfsState& st, cudaStream_t s, int sms,
-                      int32_t* d_levels);
 // has_edge for every vertex (bfs.hpp:167-170).
 void has_edge_all(const Graph& g, cudaStream_t s, int sms, uint8_t* d_out);
 

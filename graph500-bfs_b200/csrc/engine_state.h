@@ -55,10 +55,16 @@ struct Engine {
     g.device_bytes = (int64_t)arena.in_use();
   }
 
+  // Keeps room for the transient buffers of the calls between searches (the
+  // validation's copy of pred and flags, levels, has_edge: 14 bytes per id at
+  // most) and gives the rest of the free memory back.
+  void settle_memory() { arena.settle(uint64_t(16) * (uint64_t)g.pred_size + (1u << 20)); }
+
   // Runs a graph build; on failure every allocation of the build is released
   // and the handle is left without a graph.
   template <typename F>
   void build_guarded(F&& f) {
+    arena.hold();
     free_graph();
     const uint64_t m = arena.mark();
     try {
@@ -67,9 +73,11 @@ struct Engine {
       cudaStreamSynchronize(stream);
       cudaGetLastError();
       arena.rollback(m);
+      arena.settle(0);
       g = Graph();
       throw;
     }
+    settle_memory();
   }
 };
 

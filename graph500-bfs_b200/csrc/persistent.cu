@@ -35,7 +35,7 @@ namespace {
 constexpr unsigned kSpinLimit = 1u << 25;
 
 struct Shared {
-  long long level, visited, prev_nq, nq, in_rows, in_edges;
+  long long level, visited, prev_nq, nq, in_edges;
   long long q_rows;               // rows of the level's frontier list
   int forward, next_forward, growing, cur, qcur, done, fail, stop, nrec;
   unsigned long long b_nq, b_ne, b_sc;  // the block's share of the level's counters
@@ -329,7 +329,6 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     s.level = a.root_level;
     s.visited = 1;
     s.nq = 0;
-    s.in_rows = 1;
     s.in_edges = rdeg;
     s.q_rows = r >= 0 ? 1 : 0;
     s.next_forward = s.growing = 1;
@@ -409,12 +408,10 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
       if (lead) {
         const unsigned long long now = globaltimer_ns();
         PersistRec rec;
-        rec.level = (int32_t)level;
         rec.bottom_up = forward ? 0 : 1;
-        rec.input = forward ? s.in_rows : unvisited;
-        rec.discovered = nq;
-        rec.scanned = forward ? s.in_edges : sc;
-        rec.ns = (long long)(now - stamp);
+        rec.discovered = (uint32_t)nq;
+        rec.scanned = (uint32_t)(forward ? s.in_edges : sc);
+        rec.ns = (uint32_t)min(now - stamp, 0xFFFFFFFFull);
         stamp = now;
         (nrec < kPersistRecs ? s.rec[nrec] : a.more[nrec - kPersistRecs]) = rec;
         ++nrec;
@@ -455,7 +452,6 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
       if (a.force_direction == 1) next_forward = true;
       if (a.force_direction == 2) next_forward = false;
       s.next_forward = next_forward;
-      s.in_rows = nq;
       s.q_rows = (long long)(q >> 32);
       s.in_edges = (long long)(q & 0xFFFFFFFFull);
       s.qcur = qcur ^ 1;
@@ -606,26 +602,31 @@ bool run_bfs_core_persistent(const Graph& g, BfsState& st, cudaStream_t s, int s
   memset(&rs, 0, sizeof(rs));
   int64_t bytes = 4 * st.W;
   st.levels.clear();
+  int64_t visited = 1, frontier = 1;
   for (int i = 0; i < o.nrec; ++i) {
     const PersistRec& x = i < kPersistRecs ? o.rec[i] : more[(size_t)(i - kPersistRecs)];
-    const double ms = std::max<long long>(x.ns, 1) * 1e-6;
-    int64_t b;
+    const double ms = std::max<uint32_t>(x.ns, 1) * 1e-6;
+    const int32_t level = (int32_t)(root_level + 1 + i);
+    const int64_t found = x.discovered, scanned = x.scanned;
+    const int64_t input = x.bottom_up ? st.R - visited : frontier;
+    int64_t b = 16 * input + 8 * scanned + 12 * found;
     if (x.bottom_up) {
-      b = 3 * (st.W * 4) + 16 * x.input + 8 * x.scanned + 12 * x.discovered;
+      b += 3 * (st.W * 4);
       ++rs.num_bu_levels;
-      if (x.level < 64) rs.bu_level_mask |= 1ull << x.level;
-      rs.edges_scanned_bu += x.scanned;
+      if (level < 64) rs.bu_level_mask |= 1ull << level;
+      rs.edges_scanned_bu += scanned;
       rs.bu_bytes += b;
       rs.bu_ms += ms;
     } else {
-      b = 16 * x.input + 8 * x.scanned + 12 * x.discovered;
       ++rs.num_td_levels;
-      rs.edges_scanned_td += x.scanned;
+      rs.edges_scanned_td += scanned;
       rs.td_bytes += b;
       rs.td_ms += ms;
     }
     bytes += b;
-    st.levels.push_back({x.level, x.bottom_up, x.input, x.discovered, x.scanned, b, ms});
+    visited += found;
+    frontier = found;
+    st.levels.push_back({level, (int32_t)x.bottom_up, input, found, scanned, b, ms});
   }
   rs.pred_bytes = assembly_bytes(st, o.visited, sparse);
   rs.pred_ms = std::max<long long>(o.pred_ns, 1) * 1e-6;
