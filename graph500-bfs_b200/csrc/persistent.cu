@@ -27,12 +27,10 @@
 #include "common.cuh"
 #include "bfs_internal.h"
 #include "search_device.cuh"
+#include "frontier.cuh"
 
 namespace b200bfs {
 namespace {
-
-// polls of the grid barrier before it gives up (well over ten seconds)
-constexpr unsigned kSpinLimit = 1u << 25;
 
 struct Shared {
   long long level, visited, prev_nq, nq, in_edges;
@@ -50,53 +48,6 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
   return t;
 }
 
-__device__ __forceinline__ unsigned load_acquire(const unsigned* p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-// All blocks of the grid.  *target counts the arrivals that end this barrier.
-// False when a block gave up waiting; every block then leaves the kernel.
-__device__ __forceinline__ bool grid_barrier(PersistCtl* ctl, unsigned* target, Shared& s) {
-  *target += gridDim.x;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(&ctl->bar, 1u);
-    unsigned n = 0;
-    while ((int)(load_acquire(&ctl->bar) - *target) < 0) {
-      if (++n == kSpinLimit || ((n & 1023u) == 0 && load_acquire(&ctl->error) != 0)) {
-        atomicExch(&ctl->error, 1u);
-        s.fail = 1;
-        break;
-      }
-    }
-    __threadfence();
-  }
-  __syncthreads();
-  return s.fail == 0;
-}
-
-// Largest i in [0, hi] with pre[i] <= t (pre[0] = 0), for the whole warp, 32
-// probes per round.
-__device__ __forceinline__ int64_t segment_search(const uint32_t* pre, int64_t hi, uint32_t t) {
-  const int lane = lane_id();
-  int64_t lo = 0;
-  while (hi - lo > 31) {
-    const int64_t step = (hi - lo + 31) / 32;
-    const int64_t probe = lo + step * lane;
-    const unsigned le = __ballot_sync(kFull, probe <= hi && pre[probe] <= t);
-    const int last = 31 - __clz(le);
-    const int64_t next = lo + step * (last + 1);  // first probe known to be > t
-    lo += step * last;
-    if (last < 31 && next <= hi) hi = next - 1;
-  }
-  const int64_t probe = lo + lane;
-  const unsigned le = __ballot_sync(kFull, probe <= hi && pre[probe] <= t);
-  return lo + (31 - __clz(le));
-}
-
 // Frontier output of a top-down level.
 struct Emit {
   int32_t* rows;
@@ -107,27 +58,6 @@ struct Emit {
   uint32_t nq;
   unsigned long long ne;
 };
-
-// Appends a warp's rows to a frontier list: lane's n rows with d adjacency
-// entries together.  One atomic on the list's (rows, entries) word gives the
-// slots and the entry offset of the first of them, so that the list carries
-// its degree prefix without a scan.  Returns the lane's slot and offset.
-__device__ __forceinline__ void reserve(PersistCounters* c, uint32_t n, uint32_t d, int64_t* slot,
-                                        uint32_t* offset, unsigned long long* rows_after) {
-  const int lane = lane_id();
-  unsigned long long x = (unsigned long long)n << 32 | d, incl = x;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned long long t = __shfl_up_sync(kFull, incl, o);
-    if (lane >= o) incl += t;
-  }
-  unsigned long long at = 0;
-  if (lane == 31) at = atomicAdd(&c->q, incl);
-  *rows_after = (at + incl) >> 32;  // lane 31
-  at = __shfl_sync(kFull, at, 31) + incl - x;
-  *slot = (int64_t)(at >> 32);
-  *offset = (uint32_t)at;
-}
 
 // Claims kPer neighbours per lane (u < 0: none) for the parents par: the
 // vertices won are counted and appended to the next frontier.  Once the
@@ -171,12 +101,13 @@ __device__ __forceinline__ void claim(const PersistArgs& a, Emit& e, Shared& s, 
   if (!__any_sync(kFull, n != 0)) return;
 #pragma unroll
   for (int o = 16; o; o >>= 1) m += __shfl_xor_sync(kFull, m, o);
-  unsigned long long ne = 0, rows;
+  unsigned long long ne = 0, after;
   if (lane_id() == 31) ne = atomicAdd(&e.c->nq_edges, m) + m;
   int64_t slot;
   uint32_t offset;
-  reserve(e.c, n, d, &slot, &offset, &rows);
-  if (lane_id() == 31 && stop_ne >= 0 && (long long)ne > stop_ne && (long long)rows > stop_nq)
+  reserve<32>(&e.c->q, n, d, &slot, &offset, &after);
+  if (lane_id() == 31 && stop_ne >= 0 && (long long)ne > stop_ne &&
+      (long long)(after >> 32) > stop_nq)
     *(volatile int*)&s.stop = 1;
 #pragma unroll
   for (int q = 0; q < kPer; ++q) {
@@ -185,69 +116,6 @@ __device__ __forceinline__ void claim(const PersistArgs& a, Emit& e, Shared& s, 
     e.pre[slot] = offset;
     ++slot;
     offset += len[q];
-  }
-}
-
-// Edge-balanced expansion of the frontier: tiles of `tile` entries (a
-// multiple of 32, as small as one warp per tile allows) of the concatenated
-// rows, 128 entries per step.  A step inside one row needs no lookup; else the
-// rows of each 32 entries are found among the next 32 list entries (a row has
-// at least one entry, so no more can start there).
-template <int kPer>
-__device__ __forceinline__ void td_level(const PersistArgs& a, Emit& e, Shared& s, int64_t gw,
-                                         int64_t nwarps, uint32_t* vis, const int32_t* rows,
-                                         const uint32_t* pre, int64_t nrows, uint32_t total,
-                                         int64_t level, long long stop_nq, long long stop_ne) {
-  const int lane = lane_id();
-  const uint32_t tile =
-      32u * (uint32_t)min((int64_t)8, max((int64_t)1, (total + 32 * nwarps - 1) / (32 * nwarps)));
-  const int64_t ntiles = ((int64_t)total + tile - 1) / tile;
-  for (int64_t t = gw; t < ntiles; t += nwarps) {
-    const uint32_t t0 = (uint32_t)(t * tile), t1 = (uint32_t)min((int64_t)total, (t + 1) * tile);
-    int64_t i = segment_search(pre, nrows - 1, t0);
-    for (uint32_t e0 = t0; e0 < t1; e0 += 32 * kPer) {
-      int32_t u[kPer], p[kPer];
-      const uint32_t seg_hi = i + 1 < nrows ? pre[i + 1] : total;
-      if (seg_hi >= t1 || seg_hi - e0 >= 32 * kPer) {
-        const int32_t src = rows[i];
-        const int64_t rb = __ldg(a.row_ptr + src) - pre[i] + e0;
-        const int32_t par = __ldg(a.inv + src);
-#pragma unroll
-        for (int q = 0; q < kPer; ++q) {
-          const uint32_t x = q * 32 + lane;
-          u[q] = e0 + x < t1 ? __ldg(a.col + rb + x) : -1;
-          p[q] = par;
-        }
-        if (seg_hi == e0 + 32 * kPer) ++i;
-      } else {
-#pragma unroll
-        for (int q = 0; q < kPer; ++q) {
-          u[q] = -1;
-          p[q] = 0;
-          const uint32_t b = e0 + q * 32;
-          if (b >= t1) continue;  // warp-uniform
-          const uint32_t st = i + lane < nrows ? pre[i + lane] : total;
-          const uint32_t x = b + lane;
-          // last row that starts at or before entry x
-          int k = 0;
-#pragma unroll
-          for (int o = 16; o; o >>= 1) {
-            const uint32_t v = __shfl_sync(kFull, st, (k + o) & 31);
-            if (v <= x) k += o;
-          }
-          const uint32_t first = __shfl_sync(kFull, st, k);
-          if (x < t1) {
-            const int32_t src = rows[i + k];
-            u[q] = __ldg(a.col + __ldg(a.row_ptr + src) + (x - first));
-            p[q] = __ldg(a.inv + src);
-          }
-          // the row of entry b + 32
-          i += __shfl_sync(kFull, k, 31);
-          if (i + 1 < nrows && pre[i + 1] <= b + 32) ++i;
-        }
-      }
-      claim<kPer>(a, e, s, vis, u, p, level, stop_nq, stop_ne);
-    }
   }
 }
 
@@ -270,7 +138,7 @@ __device__ __forceinline__ void frontier_from_bits(const PersistArgs& a, const u
     int64_t slot;
     uint32_t offset;
     unsigned long long after;
-    reserve(c, __popc(f), d, &slot, &offset, &after);
+    reserve<32>(&c->q, __popc(f), d, &slot, &offset, &after);
     for (uint32_t g = f; g; g &= g - 1) {
       const int64_t v = w * 32 + __ffs(g) - 1;
       rows[slot] = (int32_t)v;
@@ -338,7 +206,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     s.at_set = 0;
   }
   int nrec = 0;
-  bool alive = grid_barrier(ctl, &target, s);
+  bool alive = grid_barrier(&ctl->bar, &ctl->error, &target, &s.fail);
 
   while (alive) {
     if (threadIdx.x == 0) {
@@ -361,9 +229,14 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
       e.nq = 0;
       e.ne = 0;
       const bool rule = s.growing && a.force_direction == 0;
-      td_level<kPer>(a, e, s, gw, nwarps, a.vis[cur], a.rows[qcur], a.pre[qcur], s.q_rows,
-               (uint32_t)s.in_edges, level, s.prev_nq,
-               rule ? (long long)(a.nedges / a.alpha) : -1);
+      const long long stop_nq = s.prev_nq;
+      const long long stop_ne = rule ? (long long)(a.nedges / a.alpha) : -1;
+      expand_frontier<kPer>(
+          a.row_ptr, a.col, a.rows[qcur], a.pre[qcur], s.q_rows, (uint32_t)s.in_edges, gw, nwarps,
+          [&](int32_t row) { return __ldg(a.inv + row); },
+          [&](const int32_t(&u)[kPer], const int32_t(&p)[kPer]) {
+            claim<kPer>(a, e, s, a.vis[cur], u, p, level, stop_nq, stop_ne);
+          });
       if (__any_sync(kFull, e.nq != 0)) {
         const unsigned long long n = warp_add(e.nq), d = warp_add(e.ne);
         if (lane == 0) {
@@ -398,7 +271,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     }
     __syncthreads();
     if (threadIdx.x == 0) add_counters(c, s);
-    alive = grid_barrier(ctl, &target, s);
+    alive = grid_barrier(&ctl->bar, &ctl->error, &target, &s.fail);
     if (!alive) break;
     if (threadIdx.x == 0) {
       // level end: the host loop's bookkeeping and switch rule
@@ -461,7 +334,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     if (!forward && s.next_forward) {
       frontier_from_bits(a, a.vis[s.cur], a.vis[s.cur ^ 1], gw, nwarps, a.rows[s.qcur],
                          a.pre[s.qcur], c);
-      alive = grid_barrier(ctl, &target, s);
+      alive = grid_barrier(&ctl->bar, &ctl->error, &target, &s.fail);
       if (threadIdx.x == 0) {
         const unsigned long long q = __ldcg(&c->q);
         s.q_rows = (long long)(q >> 32);

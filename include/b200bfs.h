@@ -479,17 +479,18 @@ int b200bfs_server_stop(b200bfs_server* srv);
  * writes pred[nrows] (device memory, same encoding as pred above with row ids
  * as vertex ids, -1 unreached); *num_levels (host, may be NULL) receives the
  * last level, as AUTO_LEVEL.  The CSR must be symmetric (every edge stored
- * in both directions, as the engine's own CSR is): the search is bottom-up
- * only and takes any neighbour visited before a level as the parent, which
- * gives BFS levels only on an undirected graph.  Column ids outside
+ * in both directions, as the engine's own CSR is): large levels are searched
+ * bottom-up and take any neighbour visited before the level as the parent,
+ * which gives BFS levels only on an undirected graph.  Column ids outside
  * [0, nrows) are ignored.  stream is a cudaStream_t (NULL = legacy default
- * stream); the host reads a counter after every level, so the call
- * synchronises the stream once per level and returns once the search is
+ * stream); the search is one cooperative kernel and the host reads its result,
+ * so the call synchronises the stream and returns once the search is
  * complete; a stream that is being captured is refused with
  * B200BFS_ERR_INVALID before anything is enqueued.
- * It allocates nothing: its scratch (two visited bitmaps and a counter) lives
- * in one fixed device array of B200BFS_NOALLOC_MAX_ROWS / 4 bytes that every
- * GPU loading the library keeps until exit.  Graphs with more rows are
+ * It allocates nothing: its scratch (two visited bitmaps, two frontier lists
+ * and the counters) lives in one fixed device array of
+ * B200BFS_NOALLOC_MAX_ROWS / 4 bytes and 1 MiB that every GPU loading the
+ * library keeps until exit.  Graphs with more rows are
  * rejected with B200BFS_ERR_INVALID.  The first call on a device looks up
  * that array's device address.  All calls share the array: calls that overlap
  * on the GPU (other threads or streams) race and must be serialised by the
