@@ -24,6 +24,7 @@
 #include <cub/cub.cuh>
 #include "common.cuh"
 #include "corebfs.h"
+#include "row_filter.cuh"
 
 namespace b200bfs {
 namespace {
@@ -84,33 +85,41 @@ __global__ void apply_parents_kernel(const int2* __restrict__ leaves, int64_t n,
   }
 }
 
-// Live-neighbour count of live rows; 0 for removed rows.
-__global__ void core_degree_kernel(const int64_t* __restrict__ row_ptr,
-                                   const int32_t* __restrict__ col,
-                                   const uint32_t* __restrict__ live, int64_t R,
-                                   int32_t* __restrict__ cdeg, int32_t* __restrict__ flag) {
-  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const int lane = lane_id();
-  for (int64_t r = warp; r < R; r += nw) {
-    const bool alive = (live[r >> 5] >> (r & 31)) & 1u;
-    int64_t cnt = 0;
-    if (alive) {
-      const int64_t b = row_ptr[r], e = row_ptr[r + 1];
-      for (int64_t j = b + lane; j - lane < e; j += 32) {
-        bool ok = false;
-        if (j < e) {
-          const int32_t u = col[j];
-          ok = (live[u >> 5] >> (u & 31)) & 1u;
-        }
-        cnt += __popc(__ballot_sync(kFull, ok));
-      }
-    }
-    if (lane == 0) {
-      cdeg[r] = (int32_t)cnt;
-      flag[r] = alive ? 1 : 0;
-    }
+__device__ __forceinline__ bool is_live(const uint32_t* __restrict__ live, int64_t r) {
+  return (live[r >> 5] >> (r & 31)) & 1u;
+}
+
+// Live neighbours of live rows.
+struct LiveNeighbour {
+  const int32_t* col;
+  const uint32_t* live;
+  __device__ bool operator()(int64_t r, int64_t j, int64_t) const {
+    return is_live(live, r) && is_live(live, col[j]);
   }
+};
+struct AddDegree {
+  int32_t* deg;
+  __device__ void operator()(int64_t r, int64_t c) const {
+    if (c) atomicAdd(deg + r, (int32_t)c);
+  }
+};
+struct CoreRowStart {  // -1 for removed rows
+  const uint32_t* live;
+  const int32_t* newid;
+  const int64_t* crow;
+  __device__ int64_t operator()(int64_t r) const { return is_live(live, r) ? crow[newid[r]] : -1; }
+};
+struct PutCoreNeighbour {
+  const int32_t *col, *newid;
+  int32_t* ccol;
+  __device__ void operator()(int64_t at, int64_t, int64_t j) const { ccol[at] = newid[col[j]]; }
+};
+
+__global__ void live_flag_kernel(const uint32_t* __restrict__ live, int64_t R,
+                                 int32_t* __restrict__ flag) {
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < R;
+       r += (int64_t)gridDim.x * blockDim.x)
+    flag[r] = is_live(live, r) ? 1 : 0;
 }
 
 __global__ void core_lengths_kernel(const int32_t* __restrict__ cdeg,
@@ -125,32 +134,6 @@ __global__ void core_lengths_kernel(const int32_t* __restrict__ cdeg,
     len[k] = cdeg[r];
     cinv[k] = inv[r];
     cmdeg[k] = cdeg[r];
-  }
-}
-
-__global__ void core_fill_kernel(const int64_t* __restrict__ row_ptr,
-                                 const int32_t* __restrict__ col,
-                                 const uint32_t* __restrict__ live,
-                                 const int32_t* __restrict__ newid, int64_t R,
-                                 const int64_t* __restrict__ crow, int32_t* __restrict__ ccol) {
-  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const int lane = lane_id();
-  for (int64_t r = warp; r < R; r += nw) {
-    if (!((live[r >> 5] >> (r & 31)) & 1u)) continue;
-    const int64_t b = row_ptr[r], e = row_ptr[r + 1];
-    int64_t out = crow[newid[r]];
-    for (int64_t j = b + lane; j - lane < e; j += 32) {
-      bool ok = false;
-      int32_t u = 0;
-      if (j < e) {
-        u = col[j];
-        ok = (live[u >> 5] >> (u & 31)) & 1u;
-      }
-      const unsigned m = __ballot_sync(kFull, ok);
-      if (ok) ccol[out + __popc(m & ((1u << lane) - 1))] = newid[u];
-      out += __popc(m);
-    }
   }
 }
 
@@ -265,7 +248,7 @@ int64_t read_i32(const int32_t* p, cudaStream_t s) {
 }
 
 // Rebuilds the tree list (vertex, parent) from tree_parent.
-void rebuild_tree_list(DeviceArena& arena, cudaStream_t s, int sms, Graph& g) {
+void rebuild_tree_list(DeviceArena& arena, cudaStream_t s, int sms, Graph& g, bool host_copy) {
   CoreIndex& k = g.core;
   const int64_t n = g.nverts;
   const int B = 256;
@@ -279,10 +262,13 @@ void rebuild_tree_list(DeviceArena& arena, cudaStream_t s, int sms, Graph& g) {
   k.tree_list = arena_alloc<int2>(arena, cnt, "tree list");
   tree_list_kernel<<<grid_for(n, B, sms, 16), B, 0, s>>>(k.tree_parent, pos, n, k.tree_list);
   k.tree_vertices = cnt;
-  k.h_tree_parent.resize(n);
-  check_cuda(cudaMemcpyAsync(k.h_tree_parent.data(), k.tree_parent, n * 4,
-                             cudaMemcpyDeviceToHost, s),
-             "copy tree parents");
+  // the climbs read the host's copy, which the searches' preparation brings
+  if (host_copy) {
+    k.h_tree_parent.resize(n);
+    check_cuda(cudaMemcpyAsync(k.h_tree_parent.data(), k.tree_parent, n * 4,
+                               cudaMemcpyDeviceToHost, s),
+               "copy tree parents");
+  }
   check_cuda(cudaStreamSynchronize(s), "tree list");
   arena.free(f);
   arena.free(pos);
@@ -329,7 +315,10 @@ void build_core(DeviceArena& arena, cudaStream_t s, Graph& g, int sms) {
   int32_t* cdeg = deg;  // reuse: live-neighbour counts
   int32_t* flag = arena_alloc<int32_t>(arena, R + 1, "core flags");
   int32_t* newid = arena_alloc<int32_t>(arena, R + 1, "core ids");
-  core_degree_kernel<<<grid(R * 32), B, 0, s>>>(c.row_ptr, c.col, live, R, cdeg, flag);
+  RowPieces pieces = row_pieces(arena, s, sms, c.row_ptr, R);
+  check_cuda(cudaMemsetAsync(cdeg, 0, R * 4, s), "memset");
+  count_rows(s, sms, c.row_ptr, R, pieces, LiveNeighbour{c.col, live}, AddDegree{cdeg});
+  live_flag_kernel<<<grid(R), B, 0, s>>>(live, R, flag);
   check_cuda(cudaMemsetAsync(flag + R, 0, 4, s), "memset");
   exclusive_scan_i32(arena, s, flag, newid, R + 1);
   const int64_t Rc = read_i32(newid + R, s);
@@ -353,12 +342,14 @@ void build_core(DeviceArena& arena, cudaStream_t s, Graph& g, int sms) {
   check_cuda(cudaMemcpyAsync(&k2.nedges, k2.row_ptr + Rc, 8, cudaMemcpyDeviceToHost, s), "copy");
   check_cuda(cudaStreamSynchronize(s), "core size");
   k2.col = arena_alloc<int32_t>(arena, k2.nedges, "core adjacency");
-  core_fill_kernel<<<grid(R * 32), B, 0, s>>>(c.row_ptr, c.col, live, newid, R, k2.row_ptr,
-                                              k2.col);
+  fill_rows(s, sms, c.row_ptr, R, pieces, LiveNeighbour{c.col, live},
+            CoreRowStart{live, newid, k2.row_ptr}, PutCoreNeighbour{c.col, newid, k2.col});
   k2.rank = arena_alloc<int32_t>(arena, n, "core rank");
   core_rank_kernel<<<grid(n), B, 0, s>>>(c.rank, live, newid, n, k2.rank);
+  k.h_tree_parent.resize(n);  // its pages are touched while the GPU works
   check_cuda(cudaStreamSynchronize(s), "core build");
   k2.max_degree = c.max_degree;
+  free_row_pieces(arena, pieces);
   arena.free(len);
   arena.free(flag);
   arena.free(newid);
@@ -375,7 +366,7 @@ void build_core(DeviceArena& arena, cudaStream_t s, Graph& g, int sms) {
   build_first(arena, s, c, sms);
   k.enabled = true;
   k.core_vertices = Rc;
-  rebuild_tree_list(arena, s, sms, g);
+  rebuild_tree_list(arena, s, sms, g, false);
 }
 
 void free_core(DeviceArena& arena, Graph& g) {
@@ -419,7 +410,7 @@ void core_reset_unreachable(DeviceArena& arena, cudaStream_t s, int sms, Graph& 
                                                               g.core.tree_parent);
   arena.free(reach);
   arena.free(changed);
-  rebuild_tree_list(arena, s, sms, g);
+  rebuild_tree_list(arena, s, sms, g, true);
 }
 
 void core_climb(const Graph& g, int64_t root, std::vector<int64_t>& path_v,
