@@ -72,3 +72,32 @@ def test_validate_pred_arguments(built):
         e.validate_pred(1 << 12, np.full(1 << 16, -1, np.int64))
     assert ei.value.code == 1
     e.close()
+
+
+@pytest.mark.parametrize("chain", [1, 63, 64, 65, 66, 200])
+def test_long_chains_of_unknown_depth(built, chain):
+    """CoreBFS mode: tree entries whose first ancestor of known depth is as far
+    as the depth map follows in one pass, and farther; and a cycle of them,
+    whose depths stay unknown."""
+    import b200bfs
+
+    n = 300
+    i = np.arange(n)
+    edges = np.stack([i[:-1], i[1:]], 1).astype(np.int64)
+    e = b200bfs.Engine(0)
+    e.build_from_edges(edges)
+    g = O.Graph(edges)
+    pred = np.full(e.info().pred_size, -1, np.int64)
+    pred[0] = 0
+    pred[1:n] = i[:-1] | (i[1:] << 48)
+    first = n - chain  # the last `chain` vertices of the path have unknown depth
+    pred[first:n] = (first - 1 + np.arange(chain)) | np.int64(-1 << 48)
+    want = O.validate(edges, n, pred, 0, corebfs=True, nlocalverts=pred.size)
+    assert want == (0, n - 1)
+    assert e.validate_pred(0, pred, corebfs=True) == want
+    if chain >= 63:
+        pred[first] = (first + 1) | np.int64(-1 << 48)  # first <-> first + 1
+        want = O.validate(edges, n, pred, 0, corebfs=True, nlocalverts=pred.size)
+        assert want[0] > 0
+        assert e.validate_pred(0, pred, corebfs=True) == want
+    e.close()
