@@ -787,11 +787,24 @@ __global__ void batch_pool_kernel(BatchCtl* ctl, unsigned long long* planes, uin
   ctl->done = 0;
 }
 
-// Level of root k for every row (-1: not reached), from the planes.
+// Scratch of a select, in the single-source search's block counts (16 bytes
+// at least): zeroed by its first kernel.
+struct SelectScratch {
+  int missing;         // reached rows without a neighbour one level nearer
+  unsigned blocks_done;
+  unsigned long long npieces;
+};
+
+// Level of root k for every row (-1: not reached), from the planes; and the
+// start of a select: pred = -1 everywhere, counters zero.
 __global__ void batch_row_levels_kernel(const unsigned long long* __restrict__ planes, int64_t R,
-                                        int64_t nplanes, int k, int32_t* __restrict__ out) {
-  for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < R;
-       v += (int64_t)gridDim.x * blockDim.x) {
+                                        int64_t nplanes, int k, int32_t* __restrict__ out,
+                                        int64_t* __restrict__ pred, int64_t pred_size,
+                                        SelectScratch* __restrict__ scratch) {
+  const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  if (t0 == 0) *scratch = SelectScratch{0, 0u, 0ull};
+  for (int64_t v = t0; v < R; v += stride) {
     int32_t lv = -1;
     for (int64_t L = 0; L < nplanes; ++L)
       if ((planes[L * R + v] >> k) & 1ull) {
@@ -800,12 +813,9 @@ __global__ void batch_row_levels_kernel(const unsigned long long* __restrict__ p
       }
     out[v] = lv;
   }
-}
-
-__global__ void fill_minus_one_kernel(int64_t* __restrict__ p, int64_t n) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    p[i] = -1;
+  longlong2* p2 = reinterpret_cast<longlong2*>(pred);
+  for (int64_t i = t0; i < (pred_size >> 1); i += stride) p2[i] = make_longlong2(-1, -1);
+  if (t0 == 0 && (pred_size & 1)) pred[pred_size - 1] = -1;
 }
 
 // First of the neighbours col[jb, je) at level `want`, by the whole warp; -1
@@ -848,14 +858,13 @@ constexpr int kParentPiece = 2048; // rows longer than this are left to batch_pa
 // 33-root batch at SCALE 18 with every root selected and read back takes 4.0
 // instead of 33.6 ms, a 64-root batch at SCALE 24 with two roots 6.9 instead
 // of 38 ms.
-// pieces[0, cap): (row, piece) entries, count of them in *npieces; a row
+// pieces[0, cap): (row, piece) entries, scratch->npieces of them; a row
 // that does not fit is swept here.
 __global__ void __launch_bounds__(256) batch_parent_kernel(
     const int32_t* __restrict__ lv, int64_t R, const int64_t* __restrict__ row_ptr,
     const int32_t* __restrict__ col, const int32_t* __restrict__ first,
     const int32_t* __restrict__ inv, int root_row, int64_t* __restrict__ pred,
-    int2* __restrict__ pieces, int64_t cap, unsigned long long* __restrict__ npieces,
-    int* __restrict__ missing) {
+    int2* __restrict__ pieces, int64_t cap, SelectScratch* __restrict__ scratch) {
   const int lane = lane_id();
   const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -908,7 +917,7 @@ __global__ void __launch_bounds__(256) batch_parent_kernel(
       if (je - jb > kParentPiece) {
         const int64_t n = (je - jb + kParentPiece - 1) / kParentPiece;
         int64_t at = 0;
-        if (lane == 0) at = (int64_t)atomicAdd(npieces, (unsigned long long)n);
+        if (lane == 0) at = (int64_t)atomicAdd(&scratch->npieces, (unsigned long long)n);
         at = __shfl_sync(kFull, at, 0);
         const bool fits = at + n <= cap;
         // pieces reserved for a row that does not fit are marked empty
@@ -924,7 +933,7 @@ __global__ void __launch_bounds__(256) batch_parent_kernel(
     }
     if (open) {
       if (par >= 0) pred[__ldg(inv + v)] = pred_entry(__ldg(inv + par), L);
-      else if (!deferred) atomicExch(missing, 1);
+      else if (!deferred) atomicExch(&scratch->missing, 1);
     } else if (v == root_row && L >= 0) {
       const int64_t me = __ldg(inv + v);
       pred[me] = pred_entry(me, L);
@@ -935,15 +944,16 @@ __global__ void __launch_bounds__(256) batch_parent_kernel(
 // The pieces batch_parent_kernel left: a warp scans one piece of a row's
 // last entries, unless another piece of the row has found a parent by then.
 // The pieces count from the end of the row, so that they do not depend on
-// how far its lane got (the first one may overlap what the lane tried).
+// how far its lane got (the first one may overlap what the lane tried).  The
+// last block to finish looks whether every row left to the pieces found a
+// parent, and tells the host: *result is 1, or 2 if a reached row has none.
 __global__ void __launch_bounds__(256) batch_parent_piece_kernel(
     const int32_t* __restrict__ lv, const int64_t* __restrict__ row_ptr,
     const int32_t* __restrict__ col, const int32_t* __restrict__ inv, int64_t* pred,
-    const int2* __restrict__ pieces, int64_t cap,
-    const unsigned long long* __restrict__ npieces) {
+    const int2* __restrict__ pieces, int64_t cap, SelectScratch* scratch, int* result) {
   const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const int64_t n = min((int64_t)*npieces, cap);
+  const int64_t n = min((int64_t)scratch->npieces, cap);
   for (int64_t i = gw; i < n; i += nwarps) {
     const int2 x = pieces[i];
     if (x.x < 0) continue;
@@ -958,19 +968,22 @@ __global__ void __launch_bounds__(256) batch_parent_piece_kernel(
     const int32_t p = warp_find_level(lv, col, jb, je, L - 1);
     if (p >= 0 && lane_id() == 0) pred[me] = pred_entry(__ldg(inv + p), L);
   }
-}
-
-// Rows left to the pieces that none of them found a parent for.
-__global__ void batch_parent_check_kernel(const int32_t* __restrict__ inv,
-                                          const int64_t* __restrict__ pred,
-                                          const int2* __restrict__ pieces, int64_t cap,
-                                          const unsigned long long* __restrict__ npieces,
-                                          int* __restrict__ missing) {
-  const int64_t n = min((int64_t)*npieces, cap);
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    if (pieces[i].x >= 0 && pieces[i].y == 0 && pred[inv[pieces[i].x]] == -1)
-      atomicExch(missing, 1);
+  __shared__ int s_last, s_missing;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = atomicAdd(&scratch->blocks_done, 1u) == gridDim.x - 1;
+    s_missing = 0;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!s_last) return;
+  for (int64_t i = threadIdx.x; i < n; i += blockDim.x)
+    if (pieces[i].x >= 0 && pieces[i].y == 0 && __ldcg(pred + inv[pieces[i].x]) == -1)
+      s_missing = 1;
+  __syncthreads();
+  if (threadIdx.x == 0)
+    *(volatile int*)result = s_missing || *(volatile int*)&scratch->missing ? 2 : 1;
 }
 
 __global__ void set_entry_kernel(int64_t* p, int64_t i, int64_t value) { p[i] = value; }
@@ -1151,7 +1164,7 @@ void batch_allocate(DeviceArena& arena, const Graph& g, BatchState& bs) {
   bs.blk_deg = arena_alloc<int64_t>(arena, bs.nblk + 1, "batch block degrees");
   bs.ctl = arena_alloc<BatchCtl>(arena, 1, "batch control block");
   check_cuda(cudaMallocHost(&bs.hctl, sizeof(BatchCtl)), "pinned batch control");
-  check_cuda(cudaMallocHost(&bs.hdone, sizeof(int)), "pinned flag");
+  check_cuda(cudaHostAlloc(&bs.hdone, sizeof(int), cudaHostAllocMapped), "pinned flag");
   bs.d_arg = arena_alloc<BatchSetupArg>(arena, 1, "batch arguments");
   check_cuda(cudaMallocHost(&bs.h_arg, sizeof(BatchSetupArg)), "pinned batch arguments");
   bs.allocated = true;
@@ -1485,30 +1498,24 @@ void batch_select(const Graph& g, BfsState& st, const BatchState& bs, cudaStream
   const Csr& c = batch_csr(g);
   const int B = 256;
   int32_t* lv = st.queue;  // scratch of R + 1 entries (the single-source queue)
-  batch_row_levels_kernel<<<grid_for(bs.R, B, sms, 8), B, 0, s>>>(bs.planes, bs.R, bs.levels,
-                                                                 index, lv);
-  fill_minus_one_kernel<<<grid_for(st.pred_size, B, sms, 8), B, 0, s>>>(st.pred, st.pred_size);
-  // scratch of the single-source search: a flag and a count in the block
-  // counts (two entries at least), the pieces of long rows in the degree prefix
-  int* missing = reinterpret_cast<int*>(st.blk_cnt);
-  unsigned long long* npieces = reinterpret_cast<unsigned long long*>(st.blk_cnt + 1);
+  // the long rows' pieces go to the single-source search's degree prefix
+  SelectScratch* scratch = reinterpret_cast<SelectScratch*>(st.blk_cnt);
   int2* pieces = reinterpret_cast<int2*>(st.qdeg);
   const int64_t cap = st.R + 2;
-  check_cuda(cudaMemsetAsync(st.blk_cnt, 0, 2 * sizeof(int64_t), s), "memset");
   const int root_row = bs.hctl->root_row[index];
+  *bs.hdone = 0;
+  batch_row_levels_kernel<<<grid_for(std::max(bs.R, st.pred_size / 2), B, sms, 8), B, 0, s>>>(
+      bs.planes, bs.R, bs.levels, index, lv, st.pred, st.pred_size, scratch);
   batch_parent_kernel<<<grid_for(bs.R, B, sms, 8), B, 0, s>>>(
-      lv, bs.R, c.row_ptr, c.col, c.first, c.inv, root_row, st.pred, pieces, cap, npieces,
-      missing);
-  batch_parent_piece_kernel<<<sms * 8, B, 0, s>>>(lv, c.row_ptr, c.col, c.inv, st.pred, pieces,
-                                                  cap, npieces);
-  batch_parent_check_kernel<<<sms, B, 0, s>>>(c.inv, st.pred, pieces, cap, npieces, missing);
+      lv, bs.R, c.row_ptr, c.col, c.first, c.inv, root_row, st.pred, pieces, cap, scratch);
+  batch_parent_piece_kernel<<<sms * 2, B, 0, s>>>(lv, c.row_ptr, c.col, c.inv, st.pred, pieces,
+                                                  cap, scratch, bs.hdone);
   const int64_t root = bs.roots[(size_t)index];
   if (g.core.enabled)
     core_write_tree(g, st.pred, bs.path_v[(size_t)index], bs.path_e[(size_t)index], s, sms);
   else if (root_row < 0 && root >= 0 && root < st.pred_size)
     set_entry_kernel<<<1, 1, 0, s>>>(st.pred, root, pred_entry(root, 0));
-  int hmissing = 0;
-  check_cuda(cudaMemcpyAsync(&hmissing, missing, sizeof(int), cudaMemcpyDeviceToHost, s), "copy");
+  check_cuda(cudaGetLastError(), "batch select");
   check_cuda(cudaStreamSynchronize(s), "batch select");
   // pred now holds exactly this root's result; its entry vertex is the one
   // entry outside the rows of the searched graph that a later search resets
@@ -1519,7 +1526,7 @@ void batch_select(const Graph& g, BfsState& st, const BatchState& bs, cudaStream
     st.tree_clean = true;  // core_write_tree wrote every tree parent
     st.prev_path_v = bs.path_v[(size_t)index];
   }
-  if (hmissing) throw Error{B200BFS_ERR_CUDA, "batch levels without a parent one level up"};
+  if (*bs.hdone != 1) throw Error{B200BFS_ERR_CUDA, "batch levels without a parent one level up"};
 }
 
 }  // namespace b200bfs

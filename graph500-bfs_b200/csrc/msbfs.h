@@ -83,7 +83,7 @@ struct BatchState {
   int64_t* blk_deg = nullptr;
   BatchCtl* ctl = nullptr;   // device
   BatchCtl* hctl = nullptr;  // pinned mirror
-  int* hdone = nullptr;      // pinned copy of ctl->done
+  int* hdone = nullptr;      // pinned, mapped: copy of ctl->done, result of a select
   void* d_arg = nullptr;     // device copy of the batch arguments
   void* h_arg = nullptr;     // pinned staging of the batch arguments
   std::vector<cudaEvent_t> ev;
