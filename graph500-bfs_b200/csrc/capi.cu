@@ -44,8 +44,7 @@ void* DeviceArena::alloc(size_t bytes, const char* what) {
       best = i;
   if (best < kept_.size()) {
     const Block b = kept_[best];
-    kept_[best] = kept_.back();
-    kept_.pop_back();
+    kept_.erase(kept_.begin() + (int64_t)best);
     kept_bytes_ -= b.size;
     in_use_ += bytes;
     live_.push_back({b.p, bytes, b.size, seq_++});
@@ -74,25 +73,26 @@ void* DeviceArena::alloc(size_t bytes, const char* what) {
 void DeviceArena::give(const Block& b) {
   in_use_ -= b.bytes;
   if (shared_) shared_->used.fetch_sub(b.bytes);
-  if (keep_ && b.size <= limit_ && kept_bytes_ <= limit_ - b.size) {
-    kept_.push_back(b);
-    kept_bytes_ += b.size;
-  } else {
+  if (!keep_ || b.size > limit_) {
     cudaFree(b.p);
+    return;
   }
+  kept_.push_back(b);
+  kept_bytes_ += b.size;
+  while (kept_bytes_ > limit_) drop_oldest();
 }
 
-// Keeps the smallest blocks (the costliest per byte).
+void DeviceArena::drop_oldest() {
+  cudaFree(kept_.front().p);
+  kept_bytes_ -= kept_.front().size;
+  kept_.erase(kept_.begin());
+}
+
+// What is kept so far goes back: a build's blocks are of no use afterwards.
 void DeviceArena::settle(uint64_t spare) {
   std::lock_guard<std::mutex> lock(mu_);
   limit_ = spare;
-  std::sort(kept_.begin(), kept_.end(),
-            [](const Block& a, const Block& b) { return a.size < b.size; });
-  while (kept_bytes_ > limit_) {
-    cudaFree(kept_.back().p);
-    kept_bytes_ -= kept_.back().size;
-    kept_.pop_back();
-  }
+  while (!kept_.empty()) drop_oldest();
 }
 
 void DeviceArena::free(void* p) {

@@ -50,9 +50,10 @@ struct SharedBudget {
 // us and at SCALE 16 936 -> 102 (with the one-kernel search: 70 and 77 of
 // it), a new engine's graph at SCALE 20 23.2 -> 18.7 ms, SCALE 22 with
 // CoreBFS 72 -> 59, SCALE 26 861 -> 816.
-// What is kept is bounded: settle() gives all but `spare` bytes back and sets
-// that as the limit from there on; a build holds everything until its
-// settle().  An allocation that fails gives all of it back and tries again.
+// What is kept is bounded: settle() gives it all back and sets `spare` bytes
+// as the limit from there on, beyond which the oldest block goes; a build holds
+// everything until its settle().  An allocation that fails gives all of it
+// back and tries again.
 // With a budget, own or shared, every block is freed at once, so that the
 // budget bounds what the device sees and blocks may be used on any stream.
 class DeviceArena {
@@ -82,6 +83,7 @@ class DeviceArena {
     uint64_t seq;
   };
   void give(const Block& b);  // keeps or frees a block that is no longer live
+  void drop_oldest();
   uint64_t budget_;
   uint64_t in_use_ = 0;
   uint64_t seq_ = 0;
