@@ -1287,10 +1287,6 @@ void BfsState::allocate(DeviceArena& arena, const Graph& g, cudaStream_t s) {
   hsarg = &hb->sarg;
   pub_seq = 0;
   out_seq = 0;
-  pctl = arena_alloc<PersistCtl>(arena, 1, "search kernel control block");
-  queue2 = arena_alloc<int32_t>(arena, R + 1, "frontier queue");
-  prec = arena_alloc<PersistRec>(arena, std::min<int64_t>(kMaxLevel, R + 1), "level records");
-  check_cuda(cudaMemsetAsync(pctl, 0, sizeof(PersistCtl), s), "search kernel control block");
   sctl = arena_alloc<SingleCtl>(arena, 1, "search control block");
   sarg = arena_alloc<SgArg>(arena, 1, "search arguments");
   d_vis = arena_alloc<uint32_t*>(arena, 2, "bitmap pointers");
@@ -1301,6 +1297,29 @@ void BfsState::allocate(DeviceArena& arena, const Graph& g, cudaStream_t s) {
              "bitmap pointers");
   check_cuda(cudaStreamSynchronize(s), "search buffers");
   allocated = true;
+}
+
+void BfsState::allocate_persistent(DeviceArena& arena, const Graph& g, cudaStream_t s) {
+  if (pctl || g.csr.nedges >= int64_t(1) << 32) return;
+  try {
+    queue2 = arena_alloc<int32_t>(arena, R + 1, "frontier queue");
+    prec = arena_alloc<PersistRec>(arena, std::min<int64_t>(kMaxLevel, R + 1), "level records");
+    pctl = arena_alloc<PersistCtl>(arena, 1, "search kernel control block");
+  } catch (const Error& e) {
+    if (e.code != B200BFS_ERR_OOM) throw;
+    free_persistent(arena);  // the level loop needs none of them
+    return;
+  }
+  check_cuda(cudaMemsetAsync(pctl, 0, sizeof(PersistCtl), s), "search kernel control block");
+}
+
+void BfsState::free_persistent(DeviceArena& arena) {
+  arena.free(pctl);
+  arena.free(queue2);
+  arena.free(prec);
+  pctl = nullptr;
+  queue2 = nullptr;
+  prec = nullptr;
 }
 
 cudaEvent_t BfsState::event(size_t i) {
@@ -1342,12 +1361,7 @@ void BfsState::release(DeviceArena& arena) {
   if (pmap) arena.free(pmap);
   rp = nullptr;
   pmap = nullptr;
-  arena.free(pctl);
-  arena.free(queue2);
-  queue2 = nullptr;
-  arena.free(prec);
-  pctl = nullptr;
-  prec = nullptr;
+  free_persistent(arena);
   hout = dout = nullptr;
   if (hblock) cudaFreeHost(hblock);
   hblock = nullptr;
@@ -1570,7 +1584,7 @@ static Counters wait_level(BfsState& st, cudaStream_t s) {
 void run_bfs_core(const Graph& g, BfsState& st, cudaStream_t s, int sms, int64_t root,
                   int64_t root_level, int edgefactor, double alpha, double beta, int64_t* at,
                   const RunOptions& opt, b200bfs_run_stats* stats) {
-  if (use_persistent(g, opt) && run_bfs_core_persistent(g, st, s, sms, root, root_level,
+  if (st.pctl && use_persistent(g, opt) && run_bfs_core_persistent(g, st, s, sms, root, root_level,
                                                         edgefactor, alpha, beta, at, opt, stats))
     return;
   // the device-driven loop has top-down forms 1, 3, 4 and 5 and its own

@@ -138,6 +138,7 @@ struct BfsState {
   PersistOut* hout = nullptr;             // result, host-mapped (dout: device address)
   PersistOut* dout = nullptr;
   unsigned long long out_seq = 0;
+  int clusters = -1;                      // clusters of 16 blocks the device can hold, -1: not asked
   // device-driven level loop (graph mode)
   SingleCtl* sctl = nullptr;
   SingleCtl* hsctl = nullptr;             // pinned mirror
@@ -152,6 +153,11 @@ struct BfsState {
   cudaEvent_t event(size_t i);            // creates events on demand
 
   void allocate(DeviceArena& arena, const Graph& g, cudaStream_t s);
+  // What the one-kernel search needs beside the level loop's buffers (4 bytes
+  // per row and its records); without the memory for it, searches keep the
+  // level loop.
+  void allocate_persistent(DeviceArena& arena, const Graph& g, cudaStream_t s);
+  void free_persistent(DeviceArena& arena);
   void release(DeviceArena& arena);
 };
 
@@ -193,8 +199,8 @@ struct RunOptions {
   // with per-level kernel timings
   int single_graph = 0;
   // The search as one kernel (persistent.cu).  0: never (the level loop);
-  // 1: by the rule of use_persistent; 2 and 3: on every graph it can take,
-  // with 1024 or 2048 threads per SM.
+  // 1: by the rule of use_persistent; 2, 3 and 4: on every graph it can take,
+  // with 1024 or 2048 threads per SM or as one cluster of 16 blocks.
   int persistent = 1;
   double batch_alpha = 30;  // batched search: alpha used when the caller passes alpha <= 0
 };

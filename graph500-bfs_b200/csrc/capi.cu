@@ -460,6 +460,7 @@ int b200bfs_prepare(b200bfs_handle* h, int edgefactor, double alpha, double beta
       }
       if (b200bfs::use_pred_assembly(e.g, e.opt))
         b200bfs::build_pred_assembly(e.arena, e.g, e.st, e.stream, e.sms);
+      e.st.allocate_persistent(e.arena, e.g, e.stream);
     } catch (...) {
       cudaStreamSynchronize(e.stream);
       e.st.release(e.arena);
@@ -608,7 +609,7 @@ int b200bfs_set_option(b200bfs_handle* h, const char* name, int64_t value) {
       require(value >= 0 && value <= 2, B200BFS_ERR_INVALID, "force_direction must be 0..2");
       e.opt.force_direction = (int)value;
     } else if (n == "persistent") {
-      require(value >= 0 && value <= 3, B200BFS_ERR_INVALID, "persistent must be 0..3");
+      require(value >= 0 && value <= 4, B200BFS_ERR_INVALID, "persistent must be 0..4");
       e.opt.persistent = (int)value;
     } else if (n == "batch_probe") {
       require(value == 4 || value == 8 || value == 16 || value == 32 || value == 64 ||

@@ -3,11 +3,11 @@
 // On graphs whose levels take microseconds the level loop of bfs.cu is bound
 // by its launches: a search of a SCALE 20 graph is 23 kernels and eight host
 // round trips, 273 us of which the GPU works 160.  Here the whole search is
-// one cooperative kernel: its blocks, all resident, go through the levels
-// together with a grid barrier after each, every block evaluates the
-// direction rule (bfs.hpp:3413-3457) from the level's counters by itself, and
-// the pred assembly follows in the same launch.  The host launches once and
-// waits once.
+// one kernel: its blocks, all resident, go through the levels together with
+// a barrier after each (a cooperative grid, or one cluster on small graphs).
+// Every block evaluates the direction rule (bfs.hpp:3413-3457) from the level's
+// counters by itself, and the pred assembly follows in the same launch.  The
+// host launches once and waits once.
 //
 // Top-down levels claim a vertex with an OR that returns the old word, so
 // that exactly one entry wins it; the winner counts it and appends it to the
@@ -16,7 +16,7 @@
 // levels are those of the level kernels (search_device.cuh).
 //
 // us per search (16 roots, default alpha and beta), level loop -> one kernel:
-// SCALE 12 152 -> 70, 16 207 -> 77, 20 273 -> 94, 22 333 -> 151, 24 494 -> 315,
+// SCALE 12 152 -> 60, 16 207 -> 70, 20 273 -> 94, 22 333 -> 151, 24 494 -> 315,
 // 26 973 -> 856; with CoreBFS and group reordering SCALE 24 355 -> 261, 26
 // 731 -> 656.  What bounds it: on the small graphs a chain of about ten
 // dependent loads, three atomics and the barrier (2 us) per level; from
@@ -31,6 +31,19 @@
 
 namespace b200bfs {
 namespace {
+
+// The barrier between the kernel's blocks: those of one cluster (kCluster,
+// the grid is one cluster; the hardware schedules it as one) or of a
+// cooperative grid.
+template <bool kCluster>
+__device__ __forceinline__ bool blocks_barrier(PersistCtl* ctl, unsigned* target, int* fail) {
+  if (kCluster) {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    return true;
+  }
+  return grid_barrier(&ctl->bar, &ctl->error, target, fail);
+}
 
 struct Shared {
   long long level, visited, prev_nq, nq, in_edges;
@@ -164,7 +177,7 @@ __device__ __forceinline__ unsigned long long warp_add(unsigned long long x) {
   return x;
 }
 
-template <int kWords, int kPer, int kThreads, int kMinBlocks>
+template <int kWords, int kPer, int kThreads, int kMinBlocks, bool kCluster>
 __global__ void __launch_bounds__(kThreads, kMinBlocks)
     persistent_search_kernel(const __grid_constant__ PersistArgs a) {
   __shared__ Shared s;
@@ -206,7 +219,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     s.at_set = 0;
   }
   int nrec = 0;
-  bool alive = grid_barrier(&ctl->bar, &ctl->error, &target, &s.fail);
+  bool alive = blocks_barrier<kCluster>(ctl, &target, &s.fail);
 
   while (alive) {
     if (threadIdx.x == 0) {
@@ -271,7 +284,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     }
     __syncthreads();
     if (threadIdx.x == 0) add_counters(c, s);
-    alive = grid_barrier(&ctl->bar, &ctl->error, &target, &s.fail);
+    alive = blocks_barrier<kCluster>(ctl, &target, &s.fail);
     if (!alive) break;
     if (threadIdx.x == 0) {
       // level end: the host loop's bookkeeping and switch rule
@@ -334,7 +347,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     if (!forward && s.next_forward) {
       frontier_from_bits(a, a.vis[s.cur], a.vis[s.cur ^ 1], gw, nwarps, a.rows[s.qcur],
                          a.pre[s.qcur], c);
-      alive = grid_barrier(&ctl->bar, &ctl->error, &target, &s.fail);
+      alive = blocks_barrier<kCluster>(ctl, &target, &s.fail);
       if (threadIdx.x == 0) {
         const unsigned long long q = __ldcg(&c->q);
         s.q_rows = (long long)(q >> 32);
@@ -419,26 +432,64 @@ bool run_bfs_core_persistent(const Graph& g, BfsState& st, cudaStream_t s, int s
   a.edgefactor = edgefactor;
   a.force_direction = opt.force_direction;
   a.seq = ++st.out_seq;
-  // Threads per SM: 1024 with the registers the level code asks for (no
-  // spills) while a level is a few rounds of loads per warp; above, 2048
-  // threads at 32 registers, whose loads in flight are worth more than their
-  // spills.  us per search, 16 roots, 1024 / 2048 threads: SCALE 20 (R 0.6 M)
-  // 94 / 115, SCALE 22 (2.4 M) 151 / 168, SCALE 24 (8.9 M) 321 / 315, its
-  // 2-core (6.7 M) 269 / 261, SCALE 26 (33 M) 983 / 856.
-  const bool wide = opt.persistent == 3 || (opt.persistent != 2 && st.R >= (int64_t(6) << 20));
-  auto kernel = wide ? persistent_search_kernel<2, 2, 1024, 2>
-                     : persistent_search_kernel<2, 4, 1024, 1>;
-  const int threads = 1024;
-  void* params[] = {&a};
-  const cudaError_t le =
-      cudaLaunchCooperativeKernel((const void*)kernel, dim3(sms * blocks_per_sm(kernel, threads)),
-                                  dim3(threads), params, 0, s);
-  if (le == cudaErrorCooperativeLaunchTooLarge) {
-    // a part of the device only (MPS): not every block can be resident
-    cudaGetLastError();
-    return false;
+  // Up to 80 K rows: one cluster of 16 blocks, whose barrier is the hardware's
+  // (us per search, cooperative grid / cluster: SCALE 12 62.3 / 60.1, SCALE 14
+  // 67.7 / 64.5, SCALE 16 77.5 / 69.8, its 2-core 76.1 / 68.5; SCALE 18, 170 K
+  // rows, 86.5 / 95.8: 16 SMs no longer do).
+  // Else a cooperative grid.  Threads per SM: 1024 with the registers the level
+  // code asks for (no spills) while a level is a few rounds of loads per warp;
+  // from 6 M rows 2048 threads at 32 registers, whose loads in flight are worth
+  // more than their spills.  us per search, 16 roots, 1024 / 2048 threads:
+  // SCALE 20 (R 0.6 M) 94 / 115, SCALE 22 (2.4 M) 151 / 168, SCALE 24 (8.9 M)
+  // 321 / 315, its 2-core (6.7 M) 269 / 261, SCALE 26 (33 M) 983 / 856.
+  constexpr int kThreads = 1024, kCluster = 16;
+  const bool small = opt.persistent == 4 || (opt.persistent == 1 && st.R <= 80 * 1024);
+  const bool wide =
+      opt.persistent == 3 || (opt.persistent == 1 && st.R >= (int64_t(6) << 20));
+  bool launched = false;
+  if (small) {
+    auto kernel = persistent_search_kernel<2, 4, kThreads, 1, true>;
+    cudaLaunchAttribute dim;
+    dim.id = cudaLaunchAttributeClusterDimension;
+    dim.val.clusterDim.x = kCluster;
+    dim.val.clusterDim.y = dim.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kCluster);
+    cfg.blockDim = dim3(kThreads);
+    cfg.stream = s;
+    cfg.attrs = &dim;
+    cfg.numAttrs = 1;
+    if (st.clusters < 0) {
+      // 16 blocks are beyond the portable cluster size: the device has to have
+      // a group of SMs of that many
+      int n = 0;
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+              cudaSuccess ||
+          cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+      }
+      st.clusters = n;
+    }
+    if (st.clusters > 0) {
+      check_cuda(cudaLaunchKernelEx(&cfg, kernel, a), "search kernel");
+      launched = true;
+    }
   }
-  check_cuda(le, "search kernel");
+  if (!launched) {
+    auto kernel = wide ? persistent_search_kernel<2, 2, kThreads, 2, false>
+                       : persistent_search_kernel<2, 4, kThreads, 1, false>;
+    void* params[] = {&a};
+    const cudaError_t e = cudaLaunchCooperativeKernel((const void*)kernel,
+                                                      dim3(sms * blocks_per_sm(kernel, kThreads)),
+                                                      dim3(kThreads), params, 0, s);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {
+      // a part of the device only (MPS): not every block can be resident
+      cudaGetLastError();
+      return false;
+    }
+    check_cuda(e, "search kernel");
+  }
   volatile unsigned long long* flag = &st.hout->seq;
   for (unsigned long long n = 1; *flag != a.seq; ++n) {
     if ((n & 4095) == 0) {

@@ -301,10 +301,11 @@ int b200bfs_tune_engine(b200bfs_handle* h, const int64_t* roots, int num_roots, 
  * top-down forms 1, 3, 4 or 5; per-level kernel times are then not
  * recorded; 0: host loop, the default),
  * "persistent" (1: b200bfs_run searches graphs of up to 48 M rows with one
- * cooperative kernel for all levels while the form options above are at their
- * defaults, the default; 0: always the level loop; 2 and 3: the one kernel
- * with 1024 or 2048 threads per SM on every graph of less than 2^32 directed
- * entries; level and pred times are then the device's clock),
+ * kernel for all levels while the form options above are at their defaults,
+ * the default; 0: always the level loop; 2, 3 and 4: the one kernel with 1024
+ * or 2048 threads per SM or as one cluster of 16 blocks, on every graph of less
+ * than 2^32 directed entries; level and pred times are then the device's
+ * clock),
  * "batch_graph" (1: b200bfs_run_batch runs its level loop as a CUDA graph on
  * the device, 0: the host launches each level and per-level times are
  * recorded), "batch_alpha" (the alpha b200bfs_run_batch uses when given

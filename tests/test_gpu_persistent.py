@@ -1,4 +1,4 @@
-"""The one-kernel search (option "persistent" 2 and 3) against the level loop
+"""The one-kernel search (option "persistent" 2, 3 and 4) against the level loop
 (0) and the oracle: levels, auto_tuning_data, run statistics, per-level
 records and validity of parents, on graphs whose sizes, frontiers and depths
 sit at its limits."""
@@ -33,7 +33,7 @@ def _search(engine, mode, root, alpha, beta):
             [{k: v for k, v in x.items() if k != "ms"} for x in engine.level_stats()])
 
 
-def _compare(engine, g, roots, alpha=10.0, beta=14.0, modes=(2, 3), corebfs=False):
+def _compare(engine, g, roots, alpha=10.0, beta=14.0, modes=(2, 3, 4), corebfs=False):
     engine.prepare(16, alpha, beta)
     engine.run(int(roots[0]), 16, alpha, beta)  # the first search fills pred once
     for r in (int(r) for r in roots):
@@ -111,3 +111,32 @@ def test_forms_keep_the_level_loop(engine):
         engine.run(root)
         assert engine.run_stats().kernel_launches > 2
         engine.set_option(name, default)
+
+
+def test_engines_of_two_threads(built):
+    """Searches of two engines at once, on their own streams: cooperative
+    grids that each need the whole device."""
+    import threading
+
+    import b200bfs
+
+    def work(scale, out):
+        e = b200bfs.Engine(0)
+        e.generate_graph(scale, 16)
+        e.prepare(16)
+        roots = [int(r) for r in e.find_roots(4)]
+        for i in range(60):
+            r = roots[i % 4]
+            e.run(r)
+            lv = e.get_levels()
+            out.append(np.array_equal(lv, out[i % 4][0]) if i >= 4 else (lv, e.validate(r)[0]))
+        e.close()
+
+    results = [[], []]
+    threads = [threading.Thread(target=work, args=(18 + k, results[k])) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for out in results:
+        assert len(out) == 60 and all(o[1] == 0 for o in out[:4]) and all(out[4:])
