@@ -28,6 +28,7 @@
 #include "bfs_internal.h"
 #include "search_device.cuh"
 #include "frontier.cuh"
+#include "level_rule.h"
 
 namespace b200bfs {
 namespace {
@@ -45,13 +46,9 @@ __device__ __forceinline__ bool blocks_barrier(PersistCtl* ctl, unsigned* target
   return grid_barrier(&ctl->bar, &ctl->error, target, fail);
 }
 
-struct Shared {
-  long long level, visited, prev_nq, nq, in_edges;
-  long long q_rows;               // rows of the level's frontier list
-  int forward, next_forward, growing, cur, qcur, done, fail, stop, nrec;
+struct Shared : LevelState {
+  int fail, stop, nrec;
   unsigned long long b_nq, b_ne, b_sc;  // the block's share of the level's counters
-  long long at[9];                // auto_tuning_data, and the slots written
-  unsigned at_set;
   PersistRec rec[kPersistRecs];   // kept by block 0
 };
 
@@ -287,60 +284,24 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     alive = blocks_barrier<kCluster>(ctl, &target, &s.fail);
     if (!alive) break;
     if (threadIdx.x == 0) {
-      // level end: the host loop's bookkeeping and switch rule
-      const unsigned long long q = __ldcg(&c->q);
-      const long long ne = (long long)__ldcg(&c->nq_edges), sc = (long long)__ldcg(&c->scanned);
-      const long long nq = (long long)(__ldcg(&c->nq) + (q >> 32));
+      PersistCounters end;
+      end.q = __ldcg(&c->q);
+      end.nq = __ldcg(&c->nq);
+      end.nq_edges = __ldcg(&c->nq_edges);
+      end.scanned = __ldcg(&c->scanned);
+      const long long in_edges = s.in_edges;
+      level_end(s, a, end);
       if (lead) {
         const unsigned long long now = globaltimer_ns();
         PersistRec rec;
         rec.bottom_up = forward ? 0 : 1;
-        rec.discovered = (uint32_t)nq;
-        rec.scanned = (uint32_t)(forward ? s.in_edges : sc);
+        rec.discovered = (uint32_t)s.nq;
+        rec.scanned = (uint32_t)(forward ? in_edges : (long long)end.scanned);
         rec.ns = (uint32_t)min(now - stamp, 0xFFFFFFFFull);
         stamp = now;
         (nrec < kPersistRecs ? s.rec[nrec] : a.more[nrec - kPersistRecs]) = rec;
         ++nrec;
       }
-      s.nq = nq;
-      s.visited += nq;
-      if (!forward) s.cur = cur ^ 1;
-      bool next_forward = s.next_forward != 0;
-      if (nq == 0) {
-        s.done = 1;
-      } else if (s.growing && nq > s.prev_nq) {
-        if (forward) {
-          if (ne > (long long)(a.nedges / a.alpha)) {
-            next_forward = false;
-            s.at[0] = ne;        // AUTO_GLOBAL_NQ_EDGES
-            s.at[1] = a.nedges;  // AUTO_NUM_GLOBAL_EDGES
-            s.at[2] = level;     // AUTO_T2B_LEVEL
-            s.at_set |= 7u;
-          } else {
-            s.at[6] = ne;  // AUTO_PRE_GLOBAL_NQ_EDGES
-            s.at_set |= 1u << 6;
-          }
-        }
-      } else if (!forward) {
-        if (nq < (long long)(a.R / (a.beta * a.edgefactor * 2.0))) {
-          next_forward = true;
-          s.growing = 0;
-          s.at[3] = nq;     // AUTO_GLOBAL_NQ_SIZE
-          s.at[4] = a.R;    // AUTO_NUM_GLOBAL_VERTS
-          s.at[5] = level;  // AUTO_B2T_LEVEL
-          s.at_set |= 7u << 3;
-        } else {
-          s.at[7] = nq;  // AUTO_PRE_GLOBAL_NQ_SIZE
-          s.at_set |= 1u << 7;
-        }
-      }
-      if (s.done == 0 && level >= kMaxLevel) s.done = 3;
-      if (a.force_direction == 1) next_forward = true;
-      if (a.force_direction == 2) next_forward = false;
-      s.next_forward = next_forward;
-      s.q_rows = (long long)(q >> 32);
-      s.in_edges = (long long)(q & 0xFFFFFFFFull);
-      s.qcur = qcur ^ 1;
     }
     __syncthreads();
     if (s.done) break;

@@ -1,0 +1,76 @@
+"""The end of a level in the one-kernel search, which every block evaluates
+for itself (csrc/level_rule.h), run for many blocks on the host: they have to
+agree whatever the order in which they come out of the barrier."""
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "graph500-bfs_b200", "csrc")
+NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
+
+PROGRAM = r"""
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include "level_rule.h"
+using namespace b200bfs;
+
+// A bottom-up level of `found` vertices with `entries` entries ends.  Each of
+// 148 blocks evaluates the rule; the ones that go back to top-down append
+// their share of the frontier at once, before the next block reads.
+int main(int argc, char** argv) {
+  const long long R = atoll(argv[1]), found = atoll(argv[2]), entries = atoll(argv[3]);
+  const int blocks = 148;
+  PersistArgs a;
+  memset(&a, 0, sizeof(a));
+  a.R = R;
+  a.nedges = 32 * R;
+  a.alpha = 10;
+  a.beta = 14;
+  a.edgefactor = 16;
+  PersistCounters c;
+  memset(&c, 0, sizeof(c));
+  c.nq = found;
+  LevelState first;
+  int differ = 0;
+  for (int b = 0; b < blocks; ++b) {
+    LevelState s;
+    memset(&s, 0, sizeof(s));
+    s.level = 5;
+    s.visited = R - 2 * found;
+    s.prev_nq = 8 * found;
+    s.growing = 1;
+    level_end(s, a, c);
+    if (s.next_forward)
+      c.q += (unsigned long long)(found / blocks) << 32 | (unsigned long long)(entries / blocks);
+    if (b == 0) first = s;
+    differ += s.nq != first.nq || s.visited != first.visited || s.done != first.done ||
+              s.next_forward != first.next_forward || s.growing != first.growing ||
+              s.cur != first.cur || s.qcur != first.qcur || s.at_set != first.at_set ||
+              memcmp(s.at, first.at, sizeof(s.at));
+  }
+  printf("%d %lld %lld %d\n", differ, first.nq, first.visited, first.next_forward);
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def program(tmp_path_factory):
+    d = tmp_path_factory.mktemp("level_rule")
+    src = d / "level_rule.cu"
+    src.write_text(PROGRAM)
+    subprocess.run([NVCC, "-std=c++17", "-I", CSRC, "-o", str(d / "level_rule"), str(src)],
+                   check=True)
+    return str(d / "level_rule")
+
+
+# few vertices; just below the switch (R / (14 * 16 * 2) = 2232); at it, where
+# the search stays bottom-up
+@pytest.mark.parametrize("found,forward", [(148, 1), (1500, 1), (2231, 1), (2232, 0), (9000, 0)])
+def test_blocks_agree_after_a_bottom_up_level(program, found, forward):
+    r = 1000000
+    out = subprocess.run([program, str(r), str(found), str(20 * found)], check=True,
+                         capture_output=True, text=True).stdout.split()
+    assert [int(x) for x in out] == [0, found, r - found, forward]
