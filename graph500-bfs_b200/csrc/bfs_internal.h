@@ -51,7 +51,8 @@ struct PersistCounters {         // of one level
   unsigned long long scanned;    // adjacency entries read bottom-up
 };
 struct PersistCtl {              // zero between searches
-  unsigned bar, blocks_done, error, pad;
+  unsigned bar, blocks_done, error;
+  unsigned done;                 // of PersistOut, as the first block left the levels
   unsigned long long stamp;      // when the assembly began
   PersistCounters c[3];          // of level L: c[L % 3]
 };

@@ -69,4 +69,11 @@ __host__ __device__ __forceinline__ void level_end(LevelState& s, const PersistA
   s.qcur ^= 1;
 }
 
+// What the last block to finish publishes.  A block that gave up waiting left
+// without its share of the level or of the assembly, even if the blocks it
+// waited for arrived right after and went on to the end.
+__host__ __device__ __forceinline__ int published_status(unsigned done, unsigned error) {
+  return error ? 4 : (int)done;
+}
+
 }  // namespace b200bfs

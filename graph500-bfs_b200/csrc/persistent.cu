@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
       a.out->level = s.level;
       a.out->visited = s.visited;
       a.out->nrec = nrec;
-      a.out->done = alive ? s.done : 4;
+      ctl->done = alive ? s.done : 4;
       a.out->at_set = s.at_set | 1u << 8;
       s.at[8] = s.level;  // AUTO_LEVEL
       for (int i = 0; i < 9; ++i) a.out->at[i] = s.at[i];
@@ -343,6 +343,8 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     __threadfence();
     if (atomicAdd(&ctl->blocks_done, 1u) == gridDim.x - 1) {
       __threadfence_system();
+      a.out->done = published_status(*(volatile unsigned*)&ctl->done,
+                                     *(volatile unsigned*)&ctl->error);
       a.out->pred_ns = (long long)(globaltimer_ns() - *(volatile unsigned long long*)&ctl->stamp);
       memset((void*)ctl, 0, sizeof(*ctl));
       __threadfence_system();
@@ -464,6 +466,11 @@ bool run_bfs_core_persistent(const Graph& g, BfsState& st, cudaStream_t s, int s
   }
   std::atomic_thread_fence(std::memory_order_acquire);
   const PersistOut& o = *st.hout;
+  if (o.done != 1) {
+    // pred may hold a part of this search: the next one writes all of it
+    st.assembled = false;
+    st.pred_clean = false;
+  }
   if (o.done == 3) throw Error{B200BFS_ERR_OVERFLOW, "more than 0xFFFE BFS levels"};
   if (o.done != 1) throw Error{B200BFS_ERR_TIMEOUT, "search kernel gave up waiting for its blocks"};
   st.asm_ev = -1;

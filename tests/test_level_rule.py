@@ -17,10 +17,24 @@ PROGRAM = r"""
 #include "level_rule.h"
 using namespace b200bfs;
 
+// The last barrier: block `late` reaches its poll limit just before the last
+// arrival, the others go on and the first block has a finished search.
+int last_barrier(int late) {
+  PersistCtl ctl;
+  memset(&ctl, 0, sizeof(ctl));
+  for (int b = 0; b < 148; ++b) {
+    if (b == late) ctl.error = 1;
+    if (b == 0) ctl.done = b == late ? 4 : 1;
+  }
+  printf("%d\n", published_status(ctl.done, ctl.error));
+  return 0;
+}
+
 // A bottom-up level of `found` vertices with `entries` entries ends.  Each of
 // 148 blocks evaluates the rule; the ones that go back to top-down append
 // their share of the frontier at once, before the next block reads.
 int main(int argc, char** argv) {
+  if (argc == 2) return last_barrier(atoi(argv[1]));
   const long long R = atoll(argv[1]), found = atoll(argv[2]), entries = atoll(argv[3]);
   const int blocks = 148;
   PersistArgs a;
@@ -74,3 +88,9 @@ def test_blocks_agree_after_a_bottom_up_level(program, found, forward):
     out = subprocess.run([program, str(r), str(found), str(20 * found)], check=True,
                          capture_output=True, text=True).stdout.split()
     assert [int(x) for x in out] == [0, found, r - found, forward]
+
+
+@pytest.mark.parametrize("late,status", [(-1, 1), (0, 4), (1, 4), (147, 4)])
+def test_a_block_that_gave_up_is_published(program, late, status):
+    out = subprocess.run([program, str(late)], check=True, capture_output=True, text=True).stdout
+    assert int(out) == status
