@@ -64,11 +64,13 @@ struct Scratch {
 };
 static __device__ __align__(256) Scratch g_noalloc_scratch;
 
+// A device's array and the mutex that a search holds from its launch until it
+// is complete: overlapping searches would share the barrier's count and read
+// each other's frontier lists, whose rows may be beyond their own graph.
 struct DeviceScratch {
-  bool ready = false;
+  std::mutex mu;
   Scratch* ptr = nullptr;
 };
-std::mutex g_mu;
 DeviceScratch g_scratch[256];
 
 struct Shared {
@@ -339,9 +341,9 @@ extern "C" int b200bfs_bfs_noalloc(const int64_t* row_ptr, const int32_t* col, i
   if (root < 0 || root >= nrows) return B200BFS_ERR_INVALID;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   {
-    // The per-level readback and synchronisation are not allowed during
-    // stream capture: refuse before enqueuing anything, so that the caller's
-    // capture stays intact.
+    // The read-back of the result and the synchronisation are not allowed
+    // during stream capture: refuse before enqueuing anything, so that the
+    // caller's capture stays intact.
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
       cudaGetLastError();
@@ -354,22 +356,19 @@ extern "C" int b200bfs_bfs_noalloc(const int64_t* row_ptr, const int32_t* col, i
     cudaGetLastError();
     return B200BFS_ERR_CUDA;
   }
-  Scratch* scratch = nullptr;
-  {
+  DeviceScratch& ds = g_scratch[dev];
+  std::lock_guard<std::mutex> lk(ds.mu);
+  if (!ds.ptr) {
     // Once per device, with that device current: the host-side name of the
     // array is not a device address, so fetch the address the kernels use.
-    std::lock_guard<std::mutex> lk(g_mu);
-    if (!g_scratch[dev].ready) {
-      void* p = nullptr;
-      if (cudaGetSymbolAddress(&p, g_noalloc_scratch) != cudaSuccess || !p) {
-        cudaGetLastError();
-        return B200BFS_ERR_CUDA;
-      }
-      g_scratch[dev].ptr = static_cast<Scratch*>(p);
-      g_scratch[dev].ready = true;
+    void* p = nullptr;
+    if (cudaGetSymbolAddress(&p, g_noalloc_scratch) != cudaSuccess || !p) {
+      cudaGetLastError();
+      return B200BFS_ERR_CUDA;
     }
-    scratch = g_scratch[dev].ptr;
+    ds.ptr = static_cast<Scratch*>(p);
   }
+  Scratch* scratch = ds.ptr;
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   void* params[] = {&row_ptr, &col, &nrows, &root, &pred, &scratch};

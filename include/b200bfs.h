@@ -493,9 +493,8 @@ int b200bfs_server_stop(b200bfs_server* srv);
  * B200BFS_NOALLOC_MAX_ROWS / 4 bytes and 1 MiB that every GPU loading the
  * library keeps until exit.  Graphs with more rows are
  * rejected with B200BFS_ERR_INVALID.  The first call on a device looks up
- * that array's device address.  All calls share the array: calls that overlap
- * on the GPU (other threads or streams) race and must be serialised by the
- * caller. */
+ * that array's device address.  All calls share the array: a call waits until
+ * another thread's search on the same device is complete. */
 int b200bfs_bfs_noalloc(const int64_t* row_ptr, const int32_t* col, int64_t nrows,
                         int64_t root, int64_t* pred, void* stream, int32_t* num_levels);
 

@@ -125,3 +125,43 @@ def test_path_and_grid(built):
                             np.stack([x[1:].ravel(), x[:-1].ravel()], 1)])
     row_ptr, col = _csr(edges, x.size)
     _check(row_ptr, col, [0, 4321])
+
+
+def test_calls_of_several_threads(built):
+    """Searches of graphs of unlike sizes from four threads at once, each on a
+    stream of its own: they share the library's one scratch array."""
+    import threading
+
+    import torch
+    import b200bfs
+
+    graphs, errors = [], []
+    for k in range(4):
+        rng = np.random.default_rng(k)
+        n = [70001, 300, 9001, 33][k]
+        row_ptr, col = _csr(rng.integers(0, n, (6 * n, 2)), n, rng)
+        root = int(np.diff(row_ptr).argmax())
+        graphs.append((row_ptr, col, root, _levels(row_ptr, col, root)))
+
+    def work(row_ptr, col, root, want):
+        try:
+            stream = torch.cuda.Stream()
+            with torch.cuda.stream(stream):
+                d_row, d_col = torch.from_numpy(row_ptr).cuda(), torch.from_numpy(col).cuda()
+                d_pred = torch.empty(want.size, dtype=torch.int64, device="cuda")
+            for _ in range(100):
+                with torch.cuda.stream(stream):
+                    d_pred.fill_(7)
+                depth = b200bfs.bfs_noalloc(d_row.data_ptr(), d_col.data_ptr(), want.size, root,
+                                            d_pred.data_ptr(), stream.cuda_stream)
+                assert depth == want.max() + 1
+                assert np.array_equal(d_pred.cpu().numpy() >> 48, want)
+        except BaseException as e:
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=g) for g in graphs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
