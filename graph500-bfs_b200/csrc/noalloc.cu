@@ -79,6 +79,11 @@ struct Shared {
   unsigned long long b_nq;
 };
 
+// Entries of row v; none where the row pointers decrease.
+__device__ __forceinline__ long long row_entries(const int64_t* __restrict__ row_ptr, int64_t v) {
+  return max((long long)(row_ptr[v + 1] - row_ptr[v]), 0ll);
+}
+
 // Bottom-up level: bitmap words w of 32 vertices per warp.  A lane tries up to
 // 16 neighbours, four loads at a time, then the warp sweeps the rest of its
 // row, 128 at a time.  Ids outside [0, n) are ignored rather than read out of
@@ -166,7 +171,7 @@ __device__ __forceinline__ void list_new(const int64_t* __restrict__ row_ptr, in
     if (!f) continue;
     const int64_t v = w * 32 + lane;
     const long long len =
-        ((f >> lane) & 1u) ? min((long long)(row_ptr[v + 1] - row_ptr[v]), kLongRow) : 0;
+        ((f >> lane) & 1u) ? min(row_entries(row_ptr, v), kLongRow) : 0;
     int64_t slot;
     uint32_t offset;
     unsigned long long after;
@@ -202,7 +207,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   // vertices of one that come back to top-down
   const long long entries = row_ptr[n];
   const long long most = min(entries / 14, kLongRow - 1), few = n / (14 * 32);
-  const long long rdeg = row_ptr[root + 1] - row_ptr[root];
+  const long long rdeg = row_entries(row_ptr, root);
   if (t0 == 0) {
     sc->rows[0][0] = (int32_t)root;
     sc->pre[0][0] = 0;
@@ -253,7 +258,7 @@ __global__ void __launch_bounds__(kThreads, 1)
               if (stopped) continue;
               // a row too long for the prefix ends the list: its length alone
               // sends the next level bottom-up
-              len[q] = (uint32_t)min((long long)(row_ptr[u[q] + 1] - row_ptr[u[q]]), kLongRow);
+              len[q] = (uint32_t)min(row_entries(row_ptr, u[q]), kLongRow);
               m += len[q] > 0;
               d += len[q];
             }

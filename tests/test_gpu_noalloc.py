@@ -116,6 +116,21 @@ def test_ids_out_of_range_are_ignored(built):
     _check(row_ptr, col, [0, 17, n - 1])
 
 
+def test_decreasing_row_pointers_are_empty_rows(built):
+    """Row v ends before it begins: it has no entries, as root as well.  The
+    entries it reaches back over are ignored ids, which the next row has too."""
+    rng = np.random.default_rng(6)
+    n, v = 2001, 1000
+    edges = rng.integers(0, n, (5 * n, 2))
+    row_ptr, col = _csr(edges[(edges != v).all(axis=1)], n, rng)
+    at = row_ptr[v]
+    col = np.concatenate([col[:at], np.full(5, -1, np.int32), col[at:]])
+    row_ptr[v:] += 5
+    row_ptr[v + 1] -= 5
+    assert row_ptr[v + 1] < row_ptr[v]
+    _check(row_ptr, col, [v, 0, v - 1, v + 1])
+
+
 def test_path_and_grid(built):
     i = np.arange(5000)
     row_ptr, col = _csr(np.stack([i[:-1], i[1:]], 1), 5000)
