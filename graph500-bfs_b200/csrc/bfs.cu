@@ -1300,7 +1300,7 @@ void BfsState::allocate(DeviceArena& arena, const Graph& g, cudaStream_t s) {
 }
 
 void BfsState::allocate_persistent(DeviceArena& arena, const Graph& g, cudaStream_t s) {
-  if (pctl || g.csr.nedges >= int64_t(1) << 32) return;
+  if (pctl || g.csr.nedges > kPersistEntries) return;
   try {
     queue2 = arena_alloc<int32_t>(arena, R + 1, "frontier queue");
     prec = arena_alloc<PersistRec>(arena, std::min<int64_t>(kMaxLevel, R + 1), "level records");

@@ -56,10 +56,13 @@ struct PersistCtl {              // zero between searches
   unsigned long long stamp;      // when the assembly began
   PersistCounters c[3];          // of level L: c[L % 3]
 };
-struct PersistRec {              // of one level; the graph has less than 2^32 entries
+struct PersistRec {              // of one level
   uint32_t bottom_up, discovered, scanned, ns;
 };
 constexpr int kPersistRecs = 64;  // level records published with the result
+// Entries of the graphs it takes: a list's degree prefix is in 32 bits, and so
+// is the end of the last step of its expansion, up to 128 entries further.
+constexpr int64_t kPersistEntries = (int64_t(1) << 32) - 256;
 struct PersistOut {              // host-mapped
   long long level, visited, pred_ns, at[9];
   int nrec, done;                // done: 1 finished, 3 too many levels, 4 gave up
@@ -222,7 +225,7 @@ void levels_from_pred(const BfsState& st, cudaStream_t s, int sms, int32_t* d_le
 inline bool use_pred_assembly(const Graph&, const RunOptions& o) { return o.pred_assemble != 0; }
 // Whether a search goes to the one kernel.  It has its own level code, so
 // options that pick a form of the level loop keep the level loop.  Its
-// frontier lists keep degree prefixes in 32 bits.  Its top-down levels count
+// frontier lists keep degree prefixes in 32 bits (kPersistEntries).  Its top-down levels count
 // the vertices they claim by their returning OR, where the level loop counts
 // them in a pass over the bitmaps: dearer on the levels that claim tens of
 // millions of vertices, which from SCALE 27 on outweighs the launches saved
@@ -230,7 +233,7 @@ inline bool use_pred_assembly(const Graph&, const RunOptions& o) { return o.pred
 // 2243 / 2488 plain and 1567 / 1567 with CoreBFS; 33 M and 63 M rows).
 inline bool use_persistent(const Graph& g, const RunOptions& o) {
   if (o.persistent == 0 || !use_pred_assembly(g, o) || o.single_graph) return false;
-  if (g.csr.nedges >= int64_t(1) << 32 || !g.csr.first_pair) return false;
+  if (g.csr.nedges > kPersistEntries || !g.csr.first_pair) return false;
   if (o.persistent > 1) return true;
   const RunOptions d;
   return g.csr.nrows < int64_t(3) << 24 && o.bu_kernel == d.bu_kernel &&

@@ -91,7 +91,8 @@ __device__ __forceinline__ void reserve(unsigned long long* q, uint32_t n, uint3
 // allows) of the concatenated rows, 32 * kPer entries per step.  A step
 // inside one row needs no lookup; else the rows of each 32 entries are found
 // among the next 32 list entries (a row has at least one entry, so no more
-// can start there).  claim(u, p) gets a lane's kPer neighbours (-1: none) and
+// can start there).  total + 32 * kPer is below 2^32, so that a step's end does
+// not wrap.  claim(u, p) gets a lane's kPer neighbours (-1: none) and
 // parent(row) of their rows.
 template <int kPer, typename Parent, typename Claim>
 __device__ __forceinline__ void expand_frontier(const int64_t* __restrict__ row_ptr,

@@ -177,6 +177,7 @@ __device__ __forceinline__ unsigned long long warp_add(unsigned long long x) {
 template <int kWords, int kPer, int kThreads, int kMinBlocks, bool kCluster>
 __global__ void __launch_bounds__(kThreads, kMinBlocks)
     persistent_search_kernel(const __grid_constant__ PersistArgs a) {
+  static_assert(kPersistEntries + 32 * kPer < int64_t(1) << 32, "steps of expand_frontier");
   __shared__ Shared s;
   const int lane = lane_id();
   const int64_t t0 = (int64_t)blockIdx.x * kThreads + threadIdx.x;

@@ -304,7 +304,7 @@ int b200bfs_tune_engine(b200bfs_handle* h, const int64_t* roots, int num_roots, 
  * kernel for all levels while the form options above are at their defaults,
  * the default; 0: always the level loop; 2, 3 and 4: the one kernel with 1024
  * or 2048 threads per SM or as one cluster of 16 blocks, on every graph of less
- * than 2^32 directed entries; level and pred times are then the device's
+ * than 2^32 - 255 directed entries; level and pred times are then the device's
  * clock),
  * "batch_graph" (1: b200bfs_run_batch runs its level loop as a CUDA graph on
  * the device, 0: the host launches each level and per-level times are

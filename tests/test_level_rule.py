@@ -33,7 +33,21 @@ int last_barrier(int late) {
 // A bottom-up level of `found` vertices with `entries` entries ends.  Each of
 // 148 blocks evaluates the rule; the ones that go back to top-down append
 // their share of the frontier at once, before the next block reads.
+// Whether a graph of that many rows and entries is searched by the one kernel.
+int taken(int option, int64_t rows, int64_t entries) {
+  Graph g;
+  RunOptions o;
+  int2 pair;
+  g.csr.nrows = rows;
+  g.csr.nedges = entries;
+  g.csr.first_pair = &pair;
+  o.persistent = option;
+  printf("%d\n", use_persistent(g, o) ? 1 : 0);
+  return 0;
+}
+
 int main(int argc, char** argv) {
+  if (argc == 5) return taken(atoi(argv[2]), atoll(argv[3]), atoll(argv[4]));
   if (argc == 2) return last_barrier(atoi(argv[1]));
   const long long R = atoll(argv[1]), found = atoll(argv[2]), entries = atoll(argv[3]);
   const int blocks = 148;
@@ -94,3 +108,15 @@ def test_blocks_agree_after_a_bottom_up_level(program, found, forward):
 def test_a_block_that_gave_up_is_published(program, late, status):
     out = subprocess.run([program, str(late)], check=True, capture_output=True, text=True).stdout
     assert int(out) == status
+
+
+# a list of all entries has to be expanded without its 32-bit steps wrapping:
+# 4 * 32 entries from 2^32 at the nearest
+@pytest.mark.parametrize("option,rows,entries,want", [
+    (2, 1 << 20, 2**32 - 1, 0), (2, 1 << 20, 2**32 - 128, 0), (2, 1 << 20, 2**32 - 256, 1),
+    (1, 1 << 20, 2**32 - 1, 0), (1, 1 << 20, 1 << 25, 1), (1, 3 << 24, 1 << 25, 0),
+    (2, 3 << 24, 1 << 25, 1), (0, 1 << 20, 1 << 25, 0)])
+def test_graphs_the_one_kernel_takes(program, option, rows, entries, want):
+    out = subprocess.run([program, "taken", str(option), str(rows), str(entries)], check=True,
+                         capture_output=True, text=True).stdout
+    assert int(out) == want
