@@ -23,105 +23,6 @@ void check_cuda(cudaError_t e, const char* what) {
   }
 }
 
-void* DeviceArena::alloc(size_t bytes, const char* what) {
-  if (bytes == 0) bytes = 16;
-  std::lock_guard<std::mutex> lock(mu_);
-  if (budget_ && in_use_ + bytes > budget_)
-    throw Error{B200BFS_ERR_OOM, std::string("HBM budget exceeded allocating ") + what};
-  if (shared_) {
-    const uint64_t before = shared_->used.fetch_add(bytes);
-    if (shared_->limit && before + bytes > shared_->limit) {
-      shared_->used.fetch_sub(bytes);
-      throw Error{B200BFS_ERR_OOM, std::string("shared HBM budget exceeded allocating ") + what};
-    }
-  }
-  // a kept block that is at most an eighth too large (small ones: up to twice)
-  const size_t most = bytes < (size_t(1) << 20) ? 2 * bytes : bytes + bytes / 8;
-  size_t best = kept_.size();
-  for (size_t i = 0; i < kept_.size(); ++i)
-    if (kept_[i].size >= bytes && kept_[i].size <= most &&
-        (best == kept_.size() || kept_[i].size < kept_[best].size))
-      best = i;
-  if (best < kept_.size()) {
-    const Block b = kept_[best];
-    kept_.erase(kept_.begin() + (int64_t)best);
-    kept_bytes_ -= b.size;
-    in_use_ += bytes;
-    live_.push_back({b.p, bytes, b.size, seq_++});
-    return b.p;
-  }
-  void* p = nullptr;
-  cudaError_t e = cudaMalloc(&p, bytes);
-  if (e == cudaErrorMemoryAllocation && !kept_.empty()) {
-    cudaGetLastError();
-    for (const Block& b : kept_) cudaFree(b.p);
-    kept_.clear();
-    kept_bytes_ = 0;
-    e = cudaMalloc(&p, bytes);
-  }
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    if (shared_) shared_->used.fetch_sub(bytes);
-    throw Error{B200BFS_ERR_OOM, std::string("cudaMalloc failed for ") + what + " (" +
-                                     std::to_string(bytes) + " bytes)"};
-  }
-  in_use_ += bytes;
-  live_.push_back({p, bytes, bytes, seq_++});
-  return p;
-}
-
-void DeviceArena::give(const Block& b) {
-  in_use_ -= b.bytes;
-  if (shared_) shared_->used.fetch_sub(b.bytes);
-  if (!keep_ || b.size > limit_) {
-    cudaFree(b.p);
-    return;
-  }
-  kept_.push_back(b);
-  kept_bytes_ += b.size;
-  while (kept_bytes_ > limit_) drop_oldest();
-}
-
-void DeviceArena::drop_oldest() {
-  cudaFree(kept_.front().p);
-  kept_bytes_ -= kept_.front().size;
-  kept_.erase(kept_.begin());
-}
-
-// What is kept so far goes back: a build's blocks are of no use afterwards.
-void DeviceArena::settle(uint64_t spare) {
-  std::lock_guard<std::mutex> lock(mu_);
-  limit_ = spare;
-  while (!kept_.empty()) drop_oldest();
-}
-
-void DeviceArena::free(void* p) {
-  if (!p) return;
-  std::lock_guard<std::mutex> lock(mu_);
-  for (size_t i = 0; i < live_.size(); ++i)
-    if (live_[i].p == p) {
-      const Block b = live_[i];
-      live_[i] = live_.back();
-      live_.pop_back();
-      give(b);
-      return;
-    }
-}
-
-void DeviceArena::rollback(uint64_t m) {
-  std::lock_guard<std::mutex> lock(mu_);
-  for (size_t i = 0; i < live_.size();) {
-    if (live_[i].seq >= m) {
-      const Block b = live_[i];
-      live_[i] = live_.back();
-      live_.pop_back();
-      give(b);
-    } else {
-      ++i;
-    }
-  }
-}
-
 namespace detail_io {
 
 __global__ void pairs_to_uint2_kernel(const int64_t* __restrict__ in, int64_t n,
@@ -204,7 +105,7 @@ int b200bfs_create(const b200bfs_config* cfg, b200bfs_handle** out) {
     b200bfs::check_cuda(cudaStreamCreateWithFlags(&e.stream, cudaStreamNonBlocking), "stream");
     b200bfs::check_cuda(cudaEventCreate(&e.run_ev[0]), "event");
     b200bfs::check_cuda(cudaEventCreate(&e.run_ev[1]), "event");
-    e.arena.open();
+    e.arena.open(dev);
   });
   if (rc != B200BFS_OK) {
     delete h;

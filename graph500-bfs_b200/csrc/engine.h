@@ -50,17 +50,21 @@ struct SharedBudget {
 // us and at SCALE 16 936 -> 102 (with the one-kernel search: 70 and 77 of
 // it), a new engine's graph at SCALE 20 23.2 -> 18.7 ms, SCALE 22 with
 // CoreBFS 72 -> 59, SCALE 26 861 -> 816.
-// What is kept is bounded: settle() gives it all back and sets `spare` bytes
-// as the limit from there on, beyond which the oldest block goes; a build holds
-// everything until its settle().  An allocation that fails gives all of it
-// back and tries again.
+// What is kept is bounded: hold() and settle() set the limit, beyond which the
+// oldest block goes; settle() gives all of it back first.  An allocation that
+// fails gives all of it back, and what the other arenas on the device keep,
+// and tries again: engines do not take memory from each other.  (Freeing
+// another arena's blocks is safe: cudaFree waits for the device.)
 // With a budget, own or shared, every block is freed at once, so that the
 // budget bounds what the device sees and blocks may be used on any stream.
 class DeviceArena {
  public:
   explicit DeviceArena(uint64_t budget = 0) : budget_(budget) {}
-  void open() { keep_ = budget_ == 0 && shared_ == nullptr; }
-  void hold() { limit_ = ~uint64_t(0); }
+  ~DeviceArena();
+  DeviceArena(const DeviceArena&) = delete;
+  DeviceArena& operator=(const DeviceArena&) = delete;
+  void open(int device);
+  void hold(uint64_t limit) { limit_ = limit; }
   void settle(uint64_t spare);
   void set_shared(SharedBudget* sb) {
     settle(0);
@@ -82,6 +86,8 @@ class DeviceArena {
     size_t size;   // allocated
     uint64_t seq;
   };
+  void* try_alloc(size_t bytes, const char* what, std::string* why);
+  bool others_give_back();
   void give(const Block& b);  // keeps or frees a block that is no longer live
   void drop_oldest();
   uint64_t budget_;
@@ -90,6 +96,7 @@ class DeviceArena {
   std::vector<Block> live_, kept_;
   uint64_t kept_bytes_ = 0, limit_ = 0;
   bool keep_ = false;
+  int device_ = 0;
   SharedBudget* shared_ = nullptr;
   std::mutex mu_;
 };

@@ -55,16 +55,27 @@ struct Engine {
     g.device_bytes = (int64_t)arena.in_use();
   }
 
+  // Freed memory that a build may keep for its later steps, and an engine
+  // between its calls.  Other users of the device (a framework's allocator)
+  // cannot take it back, so both are small beside the device's 180 GB, and
+  // only graphs that are small beside it as well profit in full: up to SCALE
+  // 22 a build's transient buffers, up to SCALE 26 those of the calls.
+  static constexpr uint64_t kBuildKeep = uint64_t(2) << 30;
+  static constexpr uint64_t kCallKeep = (uint64_t(1) << 30) + (1u << 20);
+
   // Keeps room for the transient buffers of the calls between searches (the
   // validation's copy of pred and flags, levels, has_edge: 14 bytes per id at
   // most) and gives the rest of the free memory back.
-  void settle_memory() { arena.settle(uint64_t(16) * (uint64_t)g.pred_size + (1u << 20)); }
+  void settle_memory() {
+    const uint64_t spare = uint64_t(16) * (uint64_t)g.pred_size + (1u << 20);
+    arena.settle(spare < kCallKeep ? spare : kCallKeep);
+  }
 
   // Runs a graph build; on failure every allocation of the build is released
   // and the handle is left without a graph.
   template <typename F>
   void build_guarded(F&& f) {
-    arena.hold();
+    arena.hold(kBuildKeep);
     free_graph();
     const uint64_t m = arena.mark();
     try {
