@@ -36,15 +36,19 @@ void DeviceArena::open(int device) {
 
 void* DeviceArena::alloc(size_t bytes, const char* what) {
   if (bytes == 0) bytes = 16;
-  Error why{B200BFS_ERR_OOM, ""};
-  for (bool again = false;; again = true) {
-    // (the lock is not held between the tries: other arenas' are taken there)
-    if (void* p = try_alloc(bytes, what, &why.msg)) return p;
-    if (again || !others_give_back()) throw why;
-  }
+  // (the lock is not held between the tries: other arenas' are taken there,
+  // and the owner frees buffers of this one)
+  std::string why;
+  bool full = false;
+  void* p = try_alloc(bytes, what, &why, &full);
+  if (!p && full && others_give_back()) p = try_alloc(bytes, what, &why, &full);
+  if (!p && give_up_ && give_up_()) p = try_alloc(bytes, what, &why, &full);
+  if (!p) throw Error{B200BFS_ERR_OOM, why};
+  return p;
 }
 
-void* DeviceArena::try_alloc(size_t bytes, const char* what, std::string* why) {
+// Null: why, and whether the device is full (else a budget).
+void* DeviceArena::try_alloc(size_t bytes, const char* what, std::string* why, bool* full) {
   std::lock_guard<std::mutex> lock(mu_);
   if (budget_ && in_use_ + bytes > budget_) {
     *why = std::string("HBM budget exceeded allocating ") + what;
@@ -83,6 +87,7 @@ void* DeviceArena::try_alloc(size_t bytes, const char* what, std::string* why) {
   if (e != cudaSuccess) {
     cudaGetLastError();
     if (shared_) shared_->used.fetch_sub(bytes);
+    *full = true;
     *why = std::string("cudaMalloc failed for ") + what + " (" + std::to_string(bytes) + " bytes)";
     return nullptr;
   }

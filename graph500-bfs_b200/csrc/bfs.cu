@@ -1299,8 +1299,9 @@ void BfsState::allocate(DeviceArena& arena, const Graph& g, cudaStream_t s) {
   allocated = true;
 }
 
-void BfsState::allocate_persistent(DeviceArena& arena, const Graph& g, cudaStream_t s) {
-  if (pctl || g.csr.nedges > kPersistEntries) return;
+void BfsState::allocate_persistent(DeviceArena& arena, const Graph& g, const RunOptions& opt,
+                                   cudaStream_t s) {
+  if (pctl || !use_persistent(g, opt)) return;
   try {
     queue2 = arena_alloc<int32_t>(arena, R + 1, "frontier queue");
     prec = arena_alloc<PersistRec>(arena, std::min<int64_t>(kMaxLevel, R + 1), "level records");

@@ -91,6 +91,8 @@ struct PersistArgs {
   unsigned long long seq;
 };
 
+struct RunOptions;
+
 struct BfsState {
   bool allocated = false;
   int64_t R = 0, W = 0, pred_size = 0, nblk = 0;
@@ -158,9 +160,10 @@ struct BfsState {
 
   void allocate(DeviceArena& arena, const Graph& g, cudaStream_t s);
   // What the one-kernel search needs beside the level loop's buffers (4 bytes
-  // per row and its records); without the memory for it, searches keep the
-  // level loop.
-  void allocate_persistent(DeviceArena& arena, const Graph& g, cudaStream_t s);
+  // per row and its records), if the options send searches of this graph to it;
+  // without the memory for it, searches keep the level loop.
+  void allocate_persistent(DeviceArena& arena, const Graph& g, const RunOptions& opt,
+                           cudaStream_t s);
   void free_persistent(DeviceArena& arena);
   void release(DeviceArena& arena);
 };

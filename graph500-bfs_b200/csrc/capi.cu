@@ -106,6 +106,7 @@ int b200bfs_create(const b200bfs_config* cfg, b200bfs_handle** out) {
     b200bfs::check_cuda(cudaEventCreate(&e.run_ev[0]), "event");
     b200bfs::check_cuda(cudaEventCreate(&e.run_ev[1]), "event");
     e.arena.open(dev);
+    e.arena.on_full([&e] { return e.give_up_one_kernel(); });
   });
   if (rc != B200BFS_OK) {
     delete h;
@@ -361,7 +362,7 @@ int b200bfs_prepare(b200bfs_handle* h, int edgefactor, double alpha, double beta
       }
       if (b200bfs::use_pred_assembly(e.g, e.opt))
         b200bfs::build_pred_assembly(e.arena, e.g, e.st, e.stream, e.sms);
-      e.st.allocate_persistent(e.arena, e.g, e.stream);
+      e.ensure_one_kernel();
     } catch (...) {
       cudaStreamSynchronize(e.stream);
       e.st.release(e.arena);
@@ -530,6 +531,7 @@ int b200bfs_set_option(b200bfs_handle* h, const char* name, int64_t value) {
     } else {
       throw b200bfs::Error{B200BFS_ERR_INVALID, "unknown option " + n};
     }
+    if (e.prepared) e.ensure_one_kernel();
   });
 }
 

@@ -3,6 +3,7 @@
 
 #include <atomic>
 #include <cstdint>
+#include <functional>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -71,6 +72,9 @@ class DeviceArena {
     keep_ = false;
     shared_ = sb;
   }
+  // Called when an allocation fails: frees buffers that the owner can do
+  // without, false if there are none.
+  void on_full(std::function<bool()> give_up) { give_up_ = std::move(give_up); }
   void* alloc(size_t bytes, const char* what);  // throws Error
   void free(void* p);
   uint64_t mark() const { return seq_; }
@@ -86,7 +90,7 @@ class DeviceArena {
     size_t size;   // allocated
     uint64_t seq;
   };
-  void* try_alloc(size_t bytes, const char* what, std::string* why);
+  void* try_alloc(size_t bytes, const char* what, std::string* why, bool* full);
   bool others_give_back();
   void give(const Block& b);  // keeps or frees a block that is no longer live
   void drop_oldest();
@@ -97,6 +101,7 @@ class DeviceArena {
   uint64_t kept_bytes_ = 0, limit_ = 0;
   bool keep_ = false;
   int device_ = 0;
+  std::function<bool()> give_up_;
   SharedBudget* shared_ = nullptr;
   std::mutex mu_;
 };

@@ -71,6 +71,17 @@ struct Engine {
     arena.settle(spare < kCallKeep ? spare : kCallKeep);
   }
 
+  // The one-kernel search has buffers beside the level loop's, on graphs that
+  // the options send to it.  They give way to any allocation that fails (a
+  // tight budget, a full device); searches then take the level loop until the
+  // next prepare or option.
+  void ensure_one_kernel() { st.allocate_persistent(arena, g, opt, stream); }
+  bool give_up_one_kernel() {
+    if (!st.pctl) return false;
+    st.free_persistent(arena);
+    return true;
+  }
+
   // Runs a graph build; on failure every allocation of the build is released
   // and the handle is left without a graph.
   template <typename F>

@@ -247,6 +247,7 @@ int b200bfs_server_add_graph(b200bfs_server* p, int scale, int edgefactor, uint6
     ge->h = h;
     ge->edgefactor = edgefactor;
     h->e.arena.set_shared(&s.budget);
+    h->e.opt.persistent = 0;  // its searches are batches
     auto fail = [&](int code) {
       std::string msg = b200bfs_last_error(h);
       for (auto& sl : ge->slots) {

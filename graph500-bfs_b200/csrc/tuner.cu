@@ -32,6 +32,7 @@ double time_searches(Engine& e, const std::vector<int64_t>& roots, int edgefacto
                      double beta, EventPair& ev) {
   b200bfs_run_stats rs;
   int64_t at[9];
+  e.ensure_one_kernel();
   auto one = [&](int64_t root) {
     if (e.g.core.enabled)
       core_run_bfs(e.g, e.st, e.stream, e.sms, root, edgefactor, alpha, beta, at, e.opt, &rs);

@@ -125,10 +125,35 @@ static int budget() {
   return 0;
 }
 
+// buffers that the owner can do without give way to an allocation that fails,
+// for want of budget or of memory
+static int spare() {
+  g_room = 100 * M;
+  DeviceArena a(50 * M), b;
+  b.open(0);
+  b.settle(64 * M);
+  for (DeviceArena* x : {&a, &b}) {
+    void* p = x->alloc(30 * M, "spare");
+    int asked = 0;
+    x->on_full([&] {
+      ++asked;
+      if (!p) return false;
+      x->free(p);
+      p = nullptr;
+      return true;
+    });
+    CHECK(!fails(*x, 20 * M) && asked == 0);
+    CHECK(!fails(*x, x == &a ? 50 * M : 100 * M) && asked == 1);
+    CHECK(fails(*x, 101 * M) && asked == 2);
+    x->settle(0);
+  }
+  return 0;
+}
+
 int main(int, char** argv) {
-  const char* names[] = {"others", "own", "limit", "budget"};
-  int (*tests[])() = {others, own, limit, budget};
-  for (int i = 0; i < 4; ++i)
+  const char* names[] = {"others", "own", "limit", "budget", "spare"};
+  int (*tests[])() = {others, own, limit, budget, spare};
+  for (int i = 0; i < 5; ++i)
     if (!strcmp(argv[1], names[i])) return tests[i]();
   return 2;
 }
@@ -146,7 +171,7 @@ def program(tmp_path_factory):
     return str(d / "arena")
 
 
-@pytest.mark.parametrize("name", ["others", "own", "limit", "budget"])
+@pytest.mark.parametrize("name", ["others", "own", "limit", "budget", "spare"])
 def test_arena(program, name):
     p = subprocess.run([program, name], capture_output=True, text=True)
     assert p.returncode == 0, p.stdout
