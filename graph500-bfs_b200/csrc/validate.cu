@@ -56,12 +56,14 @@ __device__ __forceinline__ void max_up(unsigned long long* to, unsigned long lon
 // those of the edge pass.  An entry is looked at only if its index is in range.
 // kMap: with CoreBFS, the depth map (build_bfs_depth_map) is written to map
 // in the same pass instead of a check of the depths: entries of unknown depth
-// take that of the first ancestor with a known one, plus the steps.
+// take that of the first ancestor with a known one, plus the steps.  map may
+// be pred itself: an ancestor that has its depth already only ends the climb
+// sooner, with the same depth, and parents are not changed.
 template <bool kMap>
-__global__ void pred_checks_kernel(const int64_t* __restrict__ pred, int64_t n, int64_t root,
+__global__ void pred_checks_kernel(const int64_t* pred, int64_t n, int64_t root,
                                    const int32_t* __restrict__ rank,
                                    const int32_t* __restrict__ tp, int64_t nverts,
-                                   int64_t* __restrict__ map, Checks* __restrict__ out) {
+                                   int64_t* map, Checks* __restrict__ out) {
   unsigned long long below = 0, self = 0, bad = 0, deep = 0, top = 0, used = 0;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
@@ -83,7 +85,7 @@ __global__ void pred_checks_kernel(const int64_t* __restrict__ pred, int64_t n, 
             ++deep;
             break;
           }
-          const int64_t z = __ldg(pred + q);
+          const int64_t z = pred[q];
           const int dq = q == root ? 0 : depth_of(z);
           if (dq != 0xFFFF) {
             if (dq + up < 0xFFFF) y = with_depth(x, dq + up);
@@ -200,14 +202,16 @@ void validate_device(DeviceArena& arena, cudaStream_t s, int sms, const Graph& g
   auto grid = [&](int64_t items) { return grid_for(items, B, sms, 16); };
   if (root < 0 || root >= g.nverts) throw Error{B200BFS_ERR_INVALID, "root out of range"};
   if (!g.input_edges) throw Error{B200BFS_ERR_STATE, "input edges are not resident"};
-  // the caller's pred on the device, and with CoreBFS the depth map beside it
+  // The caller's pred on the device; with CoreBFS the depth map, in the copy's
+  // place or beside the engine's pred.
   int64_t* copy = nullptr;
   if (!on_device) {
     copy = arena_alloc<int64_t>(arena, n, "pred copy");
     check_cuda(cudaMemcpyAsync(copy, pred, n * 8, cudaMemcpyDefault, s), "copy");
     pred = copy;
   }
-  int64_t* map = corebfs ? arena_alloc<int64_t>(arena, n, "depth map") : nullptr;
+  int64_t* beside = corebfs && !copy ? arena_alloc<int64_t>(arena, n, "depth map") : nullptr;
+  int64_t* map = copy ? copy : beside;
   uint8_t* valid = arena_alloc<uint8_t>(arena, n, "pred valid");
   Checks* out = arena_alloc<Checks>(arena, 1, "validation counters");
   const int64_t* p = corebfs ? map : pred;
@@ -276,7 +280,7 @@ void validate_device(DeviceArena& arena, cudaStream_t s, int sms, const Graph& g
   *errors = err;
   arena.free(out);
   arena.free(valid);
-  arena.free(map);
+  arena.free(beside);
   arena.free(copy);
 }
 

@@ -72,6 +72,24 @@ def test_batch_beside_a_prepared_graph(built, flags):
     assert _fits(budget, [_prepare, _search, _batch], flags=flags)
 
 
+def test_validation_of_a_callers_pred(built):
+    """With CoreBFS as much as that of the engine's own: pred and its depth map
+    are one array."""
+    def validate(e):
+        assert e.validate(e.root)[0] == 0
+
+    def validate_pred(e):
+        assert e.validate_pred(e.root, e.pred, corebfs=True)[0] == 0
+
+    def search(e):
+        e.root = int(e.find_roots(1)[0])
+        e.run(e.root, 16)
+        e.pred = e.get_pred()
+
+    budget = _smallest([_prepare, search, validate], flags=1)
+    assert _fits(budget + STEP, [_prepare, search, validate_pred], flags=1)
+
+
 def test_searches_go_on_without_the_one_kernel(built):
     """After its buffers gave way the level loop searches; with room again the
     next prepare brings them back."""
