@@ -205,7 +205,10 @@ __global__ void __launch_bounds__(256) warp_sort_kernel(const int64_t* __restric
     else warp_sort<8>(raw + b, (int)n, tmp);
   }
 }
-constexpr int64_t kBitmapBytes = int64_t(256) << 20;  // of a batch
+// of a batch's bitmaps, and no more than all entries take: a second buffer of
+// that size is what sorting them elsewhere needs, so a budget that has room for
+// the one has room for the other (one row's bitmap, R / 8 bytes, is smaller)
+constexpr int64_t kBitmapBytes = int64_t(256) << 20;
 constexpr int kBitTile = 8192;                        // words per block: 32 per thread
 
 // Rows of each class: counted (list null), then listed from start[class].
@@ -562,8 +565,9 @@ void build_csr(DeviceArena& arena, cudaStream_t s, const uint2* edges, int64_t m
   const int32_t* long_list = sort_list + first[4];
   if (nlong > 0) {
     const int64_t words = (R + 31) / 32, tiles = (words + kBitTile - 1) / kBitTile;
+    const int64_t bytes = std::min(kBitmapBytes, total * 4);
     const int64_t batch =
-        std::min({nlong, std::max<int64_t>(1, kBitmapBytes / (words * 4)), (int64_t)32768});
+        std::min({nlong, std::max<int64_t>(1, bytes / (words * 4)), (int64_t)32768});
     uint32_t* bits = arena_alloc<uint32_t>(arena, batch * words, "long row bitmaps");
     int32_t* count = arena_alloc<int32_t>(arena, batch * tiles, "long row counts");
     for (int64_t i = 0; i < nlong; i += batch) {

@@ -13,14 +13,14 @@ IDS = 1 << 16  # of pred and levels, at least
 EDGES = np.random.default_rng(1).integers(0, 5000, (20000, 2))
 
 
-def _fits(budget, calls, flags=0, option=None):
+def _fits(budget, calls, flags=0, option=None, edges=EDGES):
     import b200bfs
 
     e = b200bfs.Engine(0, budget)
     try:
         if option:
             e.set_option(*option)
-        e.build_from_edges(EDGES, flags=flags)
+        e.build_from_edges(edges, flags=flags)
         for call in calls:
             call(e)
         return True
@@ -88,6 +88,19 @@ def test_validation_of_a_callers_pred(built):
 
     budget = _smallest([_prepare, search, validate], flags=1)
     assert _fits(budget + STEP, [_prepare, search, validate_pred], flags=1)
+
+
+def test_sorting_long_rows_takes_no_more_than_the_entries(built):
+    """300 hubs of 16,500 entries among 4 M vertices: their bitmaps together
+    would take four times the entries."""
+    rng = np.random.default_rng(1)
+    hubs, length, n = 300, 16500, 4000000
+    leaf = hubs + rng.integers(0, n - hubs, hubs * length)
+    leaf[:n - hubs] = np.arange(hubs, n)
+    edges = np.stack([np.repeat(np.arange(hubs), length), leaf], 1)
+    # 8 bytes per edge for the edges, for their entries and for what they are
+    # compacted to (or the bitmaps), and six arrays per id: 36 bytes
+    assert _fits(24 * len(edges) + 36 * 2**22, [], edges=edges)
 
 
 def test_searches_go_on_without_the_one_kernel(built):
