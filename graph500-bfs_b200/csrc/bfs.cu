@@ -1623,6 +1623,7 @@ void run_bfs_core(const Graph& g, BfsState& st, cudaStream_t s, int sms, int64_t
   int cur = 0;  // vis[cur] is the current visited bitmap
 
   int64_t level = root_level;
+  const int64_t t2b = t2b_limit(c.nedges, alpha), b2t = b2t_limit(c.nrows, edgefactor, beta);
   bool forward = true, next_forward = true, growing = true;
   int64_t global_nq_size = 0, global_nq_edges = 0;
   int64_t visited = 1, qsize = 1;
@@ -1756,7 +1757,7 @@ void run_bfs_core(const Graph& g, BfsState& st, cudaStream_t s, int sms, int64_t
 
     if (growing && global_nq_size > prev_nq) {
       if (forward) {
-        if (global_nq_edges > (int64_t)(c.nedges / alpha)) {
+        if (global_nq_edges > t2b) {
           next_forward = false;
           if (at) {
             at[0] = global_nq_edges;  // AUTO_GLOBAL_NQ_EDGES
@@ -1769,7 +1770,7 @@ void run_bfs_core(const Graph& g, BfsState& st, cudaStream_t s, int sms, int64_t
       }
     } else {
       if (!forward) {
-        if (global_nq_size < (int64_t)(c.nrows / (beta * edgefactor * 2.0))) {
+        if (global_nq_size < b2t) {
           next_forward = true;
           growing = false;
           if (at) {

@@ -86,8 +86,8 @@ struct PersistArgs {
   PersistOut* out;
   PersistRec* more;              // records past kPersistRecs
   int64_t root, prev_root, root_level;
-  double alpha, beta;
-  int edgefactor, force_direction, sparse, pad;
+  int64_t t2b, b2t;              // the switch rule's limits
+  int force_direction, sparse;
   unsigned long long seq;
 };
 
@@ -167,6 +167,15 @@ struct BfsState {
   void free_persistent(DeviceArena& arena);
   void release(DeviceArena& arena);
 };
+
+// Limits of the direction switch (bfs.hpp:3413-3457): adjacency entries of a
+// growing frontier that go bottom-up, and vertices of one that come back to
+// top-down.  Computed on the host for the level loop and the one kernel, so that
+// both switch alike also where the quotient does not fit (tiny alpha or beta).
+inline int64_t t2b_limit(int64_t nedges, double alpha) { return (int64_t)(nedges / alpha); }
+inline int64_t b2t_limit(int64_t nrows, int edgefactor, double beta) {
+  return (int64_t)(nrows / (beta * edgefactor * 2.0));
+}
 
 struct RunOptions {
   // Bottom-up form.  1: bu_kernel (one word per warp step); 2, 3, 4:

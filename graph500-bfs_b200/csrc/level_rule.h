@@ -34,7 +34,7 @@ __host__ __device__ __forceinline__ void level_end(LevelState& s, const PersistA
     s.done = 1;
   } else if (s.growing && nq > s.prev_nq) {
     if (forward) {
-      if (ne > (long long)(a.nedges / a.alpha)) {
+      if (ne > a.t2b) {
         next_forward = false;
         s.at[0] = ne;          // AUTO_GLOBAL_NQ_EDGES
         s.at[1] = a.nedges;    // AUTO_NUM_GLOBAL_EDGES
@@ -46,7 +46,7 @@ __host__ __device__ __forceinline__ void level_end(LevelState& s, const PersistA
       }
     }
   } else if (!forward) {
-    if (nq < (long long)(a.R / (a.beta * a.edgefactor * 2.0))) {
+    if (nq < a.b2t) {
       next_forward = true;
       s.growing = 0;
       s.at[3] = nq;       // AUTO_GLOBAL_NQ_SIZE

@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
       e.ne = 0;
       const bool rule = s.growing && a.force_direction == 0;
       const long long stop_nq = s.prev_nq;
-      const long long stop_ne = rule ? (long long)(a.nedges / a.alpha) : -1;
+      const long long stop_ne = rule ? a.t2b : -1;
       expand_frontier<kPer>(
           a.row_ptr, a.col, a.rows[qcur], a.pre[qcur], s.q_rows, (uint32_t)s.in_edges, gw, nwarps,
           [&](int32_t row) { return __ldg(a.inv + row); },
@@ -391,9 +391,8 @@ bool run_bfs_core_persistent(const Graph& g, BfsState& st, cudaStream_t s, int s
   a.prev_root = sparse ? st.prev_root : -1;
   a.sparse = sparse ? 1 : 0;
   a.root_level = root_level;
-  a.alpha = alpha;
-  a.beta = beta;
-  a.edgefactor = edgefactor;
+  a.t2b = t2b_limit(c.nedges, alpha);
+  a.b2t = b2t_limit(st.R, edgefactor, beta);
   a.force_direction = opt.force_direction;
   a.seq = ++st.out_seq;
   // Up to 80 K rows: one cluster of 16 blocks, whose barrier is the hardware's

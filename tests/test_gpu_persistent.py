@@ -52,10 +52,12 @@ def _compare(engine, g, roots, alpha=10.0, beta=14.0, modes=(2, 3, 4), corebfs=F
 
 
 @pytest.mark.parametrize("scale,flags", [(5, 0), (10, 0), (10, 3), (14, 1), (16, 2), (18, 0)])
-@pytest.mark.parametrize("alpha,beta", [(10.0, 14.0), (1e-9, 14.0), (1e9, 14.0), (30.0, 2.0)])
+@pytest.mark.parametrize("alpha,beta", [(10.0, 14.0), (1e-9, 14.0), (1e9, 14.0), (30.0, 2.0),
+                                        (1e-15, 14.0), (30.0, 1e-16)])
 def test_generated_graphs(engine, scale, flags, alpha, beta):
     """Every direction sequence: the rule, all top-down (alpha 1e-9),
-    bottom-up after level 1 (1e9) and an early return to top-down."""
+    bottom-up after level 1 (1e9), an early return to top-down, and limits of
+    the switch beyond 64 bits."""
     edges = O.generate_edges(scale)
     g = O.Graph(edges)
     engine.generate_graph(scale, 16, flags=flags)

@@ -55,9 +55,8 @@ int main(int argc, char** argv) {
   memset(&a, 0, sizeof(a));
   a.R = R;
   a.nedges = 32 * R;
-  a.alpha = 10;
-  a.beta = 14;
-  a.edgefactor = 16;
+  a.t2b = t2b_limit(a.nedges, 10);
+  a.b2t = b2t_limit(a.R, 16, 14);
   PersistCounters c;
   memset(&c, 0, sizeof(c));
   c.nq = found;
