@@ -1,6 +1,8 @@
 """CSR construction around the row lengths where its passes change: rows cut
-into pieces (2048, pieces of 4096 entries), rows sorted by bitmap (8192), with
-duplicates and self-loops, plain, group-reordered and with CoreBFS."""
+into pieces (2048, pieces of 4096 entries); rows sorted by a warp (up to 256),
+by a block (512, 2048, 8192, 16384), by bitmap (above 16384, from R / 512) and
+by the segmented sort (between the two); with duplicates and self-loops, plain,
+group-reordered and with CoreBFS."""
 import numpy as np
 import pytest
 
@@ -62,8 +64,8 @@ def test_rows(engine, degree, flags):
     assert (d[1:][inside[1:]] <= d[:-1][inside[1:]]).all()
 
 
-def test_more_long_rows_than_a_batch(engine):
-    """Complete graph on 9000 vertices: every row is long."""
+def test_complete_graph(engine):
+    """9000 vertices: every row is of the longest that a block sorts."""
     n = 9000
     a, b = np.triu_indices(n, 1)
     engine.build_from_edges(np.stack([a, b], 1).astype(np.int64))
@@ -72,3 +74,46 @@ def test_more_long_rows_than_a_batch(engine):
     c = col.reshape(n, n - 1)
     want = np.arange(n - 1)[None, :] + (np.arange(n - 1)[None, :] >= np.arange(n)[:, None])
     assert np.array_equal(c, want)
+
+
+def _same(engine, edges, n):
+    """The CSR of a list without self-loops, entry by entry, and its order."""
+    engine.build_from_edges(edges)
+    row_ptr, col, inv, mdeg = (a.astype(np.int64) for a in engine.get_csr())
+    raw = np.bincount(edges.ravel(), minlength=n)
+    want = np.unique(np.concatenate([edges[:, 0] * n + edges[:, 1],
+                                     edges[:, 1] * n + edges[:, 0]]))
+    src = np.repeat(inv, np.diff(row_ptr))
+    assert np.array_equal(np.sort(src * n + inv[col]), want)
+    assert np.array_equal(mdeg, raw[inv]) and (np.diff(mdeg) <= 0).all()
+    # row ids are in the order of the degrees, so every row is ascending
+    inside = np.ones(col.size, bool)
+    inside[row_ptr[:-1]] = False
+    assert (col[1:] > col[:-1])[inside[1:]].all()
+    return raw
+
+
+def test_more_bitmap_rows_than_a_batch(engine):
+    """150 rows of 16,500 entries, and room for the bitmaps of 132 (four bytes
+    per entry, an eighth of a byte per row of the graph)."""
+    rng = np.random.default_rng(2)
+    hubs, length, n = 150, 16500, 1200000
+    leaf = hubs + rng.integers(0, n - hubs, hubs * length)
+    leaf[:n - hubs] = np.arange(hubs, n)
+    edges = np.stack([np.repeat(np.arange(hubs), length), leaf], 1)
+    raw = _same(engine, edges[rng.permutation(len(edges))], n)
+    assert (raw > 16384).sum() * (n // 8) > 4 * raw.sum()
+
+
+def test_segmented_rows(engine):
+    """9 M rows, so that bitmaps begin at 17,578 entries: rows on both sides of
+    that and of a block's 16,384, among rows of one to a few entries."""
+    rng = np.random.default_rng(3)
+    n = 9000000
+    lengths = [16383, 16384, 16385, 16500, 17000, 17576, 17577, 17578, 17579, 20000]
+    pairs = rng.permutation(np.arange(len(lengths), n)).reshape(-1, 2)
+    hubs = [np.stack([np.full(k, h), rng.integers(len(lengths), n, k)], 1)
+            for h, k in enumerate(lengths)]
+    edges = np.concatenate([pairs] + hubs)
+    raw = _same(engine, edges[rng.permutation(len(edges))], n)
+    assert ((raw > 16384) & (raw < n // 512)).sum() == 5
