@@ -9,16 +9,13 @@ import os
 import subprocess
 import sys
 
-import pytest
+from conftest import reference_program
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def test_reference_arm_line(built):
-    exe = os.path.join(ROOT, "oracle", "_ref", "ref_runnable_group")
-    if not os.path.exists(exe):
-        pytest.fail("oracle/_ref/ref_runnable_group missing: `make -C oracle/ref` where the "
-                    "reference tree is")
+    reference_program("ref_runnable_group")
     env = dict(os.environ, OMP_NUM_THREADS=str(min(os.cpu_count() or 1, 8)))
     p = subprocess.run([sys.executable, os.path.join(ROOT, "bench.py"), "--impl", "reference",
                         "--steps", "4", "--warmup", "2", "--ref-scale", "12"],

@@ -25,12 +25,12 @@ import numpy as np
 import pytest
 
 import oracle as O
+from conftest import reference_program
 
 pytestmark = pytest.mark.gpu
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 GOLDEN = os.path.join(ROOT, "tests", "golden")
-REF_BIN = os.path.join(ROOT, "oracle", "_ref")
 FIXTURES = sorted(glob.glob(os.path.join(GOLDEN, "reference_bfs_*.npz")))
 NAMES = [os.path.basename(f)[len("reference_bfs_"):-4] for f in FIXTURES]
 
@@ -92,7 +92,7 @@ def test_engine_reproduces_reference(engine, name):
 
 def _run_driver(exe, args, timeout=600):
     env = dict(os.environ, OMP_NUM_THREADS=str(min(os.cpu_count() or 1, 16)))
-    p = subprocess.run([os.path.join(REF_BIN, exe)] + args, capture_output=True, text=True,
+    p = subprocess.run([exe] + args, capture_output=True, text=True,
                        timeout=timeout, env=env)
     assert p.returncode == 0, (p.returncode, p.stdout[-2000:], p.stderr[-2000:])
     return p.stdout + p.stderr
@@ -114,9 +114,7 @@ def _result(out):
     ("b200_runnable_group", ["20", "-C", "-n", "4"]),
 ])
 def test_reference_driver_runs_engine(built, exe, args):
-    if not os.path.exists(os.path.join(REF_BIN, exe)):
-        pytest.fail("%s missing: build it with `make -C oracle/ref` where the reference is" % exe)
-    out = _run_driver(exe, args)
+    out = _run_driver(reference_program(exe), args)
     assert "No results printed for invalid run" not in out
     res = _result(out)
     scale = int(args[0])

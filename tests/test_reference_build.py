@@ -18,19 +18,11 @@ import subprocess
 import pytest
 
 import oracle as O
+from conftest import reference_program
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-REF_BIN = os.path.join(ROOT, "oracle", "_ref")
 PROGRAMS = ["ref_runnable", "ref_runnable_group", "ref_dump", "ref_dump_group",
             "b200_runnable", "b200_runnable_group", "gen_golden"]
-
-
-def _exe(name):
-    path = os.path.join(REF_BIN, name)
-    if not os.path.exists(path):
-        pytest.fail("%s missing: build it with `make -C oracle/ref` where the reference "
-                    "tree is" % name)
-    return path
 
 
 def _result(out):
@@ -44,13 +36,13 @@ def _result(out):
 
 
 def test_shim_selftest(built):
-    p = subprocess.run([_exe("shim_selftest")], capture_output=True, text=True, timeout=60)
+    p = subprocess.run([reference_program("shim_selftest")], capture_output=True, text=True, timeout=60)
     assert p.returncode == 0 and p.stdout.strip() == "ok", p.stderr
 
 
 def test_programs_built(built):
     for name in PROGRAMS:
-        assert os.access(_exe(name), os.X_OK), name
+        assert os.access(reference_program(name), os.X_OK), name
 
 
 @pytest.mark.parametrize("exe,args", [
@@ -60,7 +52,7 @@ def test_programs_built(built):
 ])
 def test_reference_driver_validates(built, exe, args):
     env = dict(os.environ, OMP_NUM_THREADS=str(min(os.cpu_count() or 1, 8)))
-    p = subprocess.run([_exe(exe)] + args, capture_output=True, text=True, timeout=300, env=env)
+    p = subprocess.run([reference_program(exe)] + args, capture_output=True, text=True, timeout=300, env=env)
     assert p.returncode == 0, p.stderr[-2000:]
     out = p.stdout + p.stderr
     assert "No results printed for invalid run" not in out
@@ -75,7 +67,7 @@ def test_reference_driver_validates(built, exe, args):
 
 @pytest.mark.parametrize("exe", ["b200_runnable", "b200_runnable_group"])
 def test_dropin_links_engine(built, exe):
-    p = subprocess.run(["ldd", _exe(exe)], capture_output=True, text=True, timeout=60)
+    p = subprocess.run(["ldd", reference_program(exe)], capture_output=True, text=True, timeout=60)
     line = [l for l in p.stdout.splitlines() if "libb200bfs.so" in l]
     assert line, p.stdout
     assert os.path.realpath(os.path.join(ROOT, "graph500-bfs_b200", "libb200bfs.so")) in \

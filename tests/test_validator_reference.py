@@ -13,22 +13,18 @@ import numpy as np
 import pytest
 
 import oracle as O
+from conftest import reference_program
 from pred_corruptions import corruptions
-
-ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-REF_VALIDATE = os.path.join(ROOT, "oracle", "_ref", "ref_validate")
 
 
 def reference_verdicts(scale, root, corebfs, preds, tmp_path):
-    if not os.path.exists(REF_VALIDATE):
-        pytest.fail("oracle/_ref/ref_validate missing: build it with `make -C oracle/ref` "
-                    "where the reference tree is")
+    exe = reference_program("ref_validate")
     files = []
     for i, p in enumerate(preds):
         f = tmp_path / ("pred_%02d.bin" % i)
         np.ascontiguousarray(p, np.int64).tofile(f)
         files.append(str(f))
-    cmd = [REF_VALIDATE, str(scale), str(root)] + (["-C"] if corebfs else []) + files
+    cmd = [exe, str(scale), str(root)] + (["-C"] if corebfs else []) + files
     env = dict(os.environ, OMP_NUM_THREADS=str(min(os.cpu_count() or 1, 8)))
     p = subprocess.run(cmd, capture_output=True, text=True, timeout=300, env=env)
     assert p.returncode == 0, p.stderr[-2000:]
