@@ -6,12 +6,24 @@ without copies, and a config naming the SCALE and options that actually
 ran."""
 import json
 import os
+import shutil
 import subprocess
 import sys
 
 from conftest import reference_program
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+def test_reference_arm_without_the_program(tmp_path):
+    """Where the reference's program is not built: one line that says so, exit 0."""
+    shutil.copy(os.path.join(ROOT, "bench.py"), tmp_path)
+    p = subprocess.run([sys.executable, str(tmp_path / "bench.py"), "--impl", "reference",
+                        "--steps", "4", "--warmup", "3"],
+                       capture_output=True, text=True, timeout=120, cwd=tmp_path)
+    assert p.returncode == 0, p.stderr[-3000:]
+    d = json.loads(p.stdout)
+    assert d["impl"] == "reference" and "not built" in d["unavailable"] and len(d) == 2
 
 
 def test_reference_arm_line(built):
