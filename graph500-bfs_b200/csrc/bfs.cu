@@ -960,9 +960,9 @@ __device__ __forceinline__ int32_t level_of_entry(int64_t e, const int64_t* __re
 }
 
 // Four ids per thread (n is a multiple of 4; both arrays are 256-byte
-// aligned): one pass over pred and one over the levels is all that is left of
-// it (SCALE 26 with CoreBFS: 127 us, and 379 us in five further passes over
-// the tree vertices, before).
+// aligned), in one pass over pred and the levels: SCALE 26 with CoreBFS 127 us,
+// where filling in the tree vertices' levels in passes of their own takes
+// five more of 379 us together.
 __global__ void levels_kernel(const int64_t* __restrict__ pred, int64_t n,
                               int32_t* __restrict__ lv) {
   const longlong2* p2 = reinterpret_cast<const longlong2*>(pred);

@@ -19,8 +19,8 @@
 //      validity of parents, and hub-first lists let the bottom-up searches
 //      stop early.
 // Self-loops are dropped as in make_symmetry_edge_list (:409, 429, 447).
-// All passes are bandwidth-bound integer streams; CUB supplies the radix
-// sorts and scans of this (untimed) construction step.
+// Most passes are bandwidth-bound integer streams; the placement is bound by its
+// random atomics.  CUB supplies the radix sorts and scans.
 #include <algorithm>
 #include <cub/cub.cuh>
 #include "common.cuh"
@@ -151,9 +151,9 @@ __global__ void boundary_kernel(const uint64_t* __restrict__ keys, int64_t n, in
 // setting the row's keys' bits (keys are below R) and reading them back in
 // order, which drops the duplicates as well; all rows of a batch together and
 // every pass spread over the grid.  Between the two, on graphs of more than 8 M
-// rows: CUB's segmented sort.  It sorted every row before, and gives one of
-// more than some hundred entries to a block that goes through global memory
-// over all 32 bits: 10.3 ms of a SCALE 22 build, 3.4 ms now.
+// rows: CUB's segmented sort, which gives a row of more than some hundred
+// entries to a block that goes through global memory over all 32 bits.  The
+// rows of a SCALE 22 build: 10.3 ms by the segmented sort alone, 3.4 ms so.
 constexpr int kWarpRow = 256, kBlockRow = 16384;
 constexpr int kSortClasses = 6;  // 0..3 block sorts, 4 bitmap, 5 segmented sort
 __host__ __device__ __forceinline__ bool in_segmented_sort(int64_t len, int64_t long_row) {

@@ -47,10 +47,10 @@ struct SharedBudget {
 // 22 build makes 60 of those calls, about 45 of its 90 ms).  A stream-ordered
 // pool (cudaMallocFromPoolAsync) reuses as fast but maps and unmaps new
 // memory at 5-7 ms per GB, against 1 ms: first builds took 15-25 % longer.
-// Measured, before -> after: one search and its levels at SCALE 12 957 -> 93
-// us and at SCALE 16 936 -> 102 (with the one-kernel search: 70 and 77 of
-// it), a new engine's graph at SCALE 20 23.2 -> 18.7 ms, SCALE 22 with
-// CoreBFS 72 -> 59, SCALE 26 861 -> 816.
+// Measured, without -> with kept blocks: one search and its levels at SCALE 12
+// 957 -> 93 us and at SCALE 16 936 -> 102 (with the one-kernel search: 70 and
+// 77 of it), a new engine's graph at SCALE 20 23.2 -> 18.7 ms, SCALE 22 with
+// CoreBFS 72 -> 59.
 // What is kept is bounded: hold() and settle() set the limit, beyond which the
 // oldest block goes; settle() gives all of it back first.  An allocation that
 // fails gives all of it back, and what the other arenas on the device keep,

@@ -854,10 +854,10 @@ constexpr int kParentPiece = 2048; // rows longer than this are left to batch_pa
 // vertices at the end of millions of entries, are cut into pieces of
 // kParentPiece entries that a second kernel spreads over the grid.  What
 // bounds it is the longest serial scan: with a thread per row the hubs'
-// scans took 15-29 ms of a select at SCALE 24 and 0.9 ms at SCALE 18; now a
-// 33-root batch at SCALE 18 with every root selected and read back takes 4.0
-// instead of 33.6 ms, a 64-root batch at SCALE 24 with two roots 6.9 instead
-// of 38 ms.
+// scans take 15-29 ms of a select at SCALE 24 and 0.9 ms at SCALE 18.  A
+// 33-root batch at SCALE 18 with every root selected and read back: 33.6 ms
+// with a thread per row, 4.0 so; a 64-root batch at SCALE 24 with two roots:
+// 38 and 6.9 ms.
 // pieces[0, cap): (row, piece) entries, scratch->npieces of them; a row
 // that does not fit is swept here.
 __global__ void __launch_bounds__(256) batch_parent_kernel(

@@ -17,12 +17,12 @@
 // entries, or more rows than the list has room for) are searched bottom-up:
 // a warp owns 32 vertices, each unvisited one looks for a neighbour visited
 // before the level, and the next bitmap word is built with __ballot_sync.
-// Bottom-up alone is a correct BFS on a symmetric CSR too, and it was what ran
-// here before, a kernel and a readback per level: the first levels then read
-// nearly the whole CSR and waited for the warps that swept the hubs' rows
-// alone.  A SCALE 20 Kronecker graph in its own vertex order: 1,400-1,870 us
-// before, 118 us now (levels extracted by the caller included).  What bounds
-// it is the dependent loads and the barrier of each level.
+// Bottom-up alone is a correct BFS on a symmetric CSR too, with a kernel and a
+// readback per level, but its first levels read nearly the whole CSR and wait
+// for the warps that sweep the hubs' rows alone: a SCALE 20 Kronecker graph in
+// its own vertex order takes 1,400-1,870 us so and 102-118 in this form (levels
+// extracted by the caller included).  What bounds it is the dependent loads
+// and the barrier of each level.
 // The host reads the result after the kernel, so the call synchronises its
 // stream; a stream that is being captured into a CUDA graph is refused before
 // anything is enqueued on it.

@@ -51,9 +51,9 @@ __device__ __forceinline__ void max_up(unsigned long long* to, unsigned long lon
 // Value ranges, self-parents, depths and the highest used vertex
 // (find_max_used_vertex, benchmark_helper.hpp:564-582: rank or tree parent as
 // in has_edge) of every id, whichever of them the verdict turns out to need:
-// they were six passes with a readback after each, 130 us of kernels and as
-// much waiting at SCALE 23, and are one of 35 us whose counters are read with
-// those of the edge pass.  An entry is looked at only if its index is in range.
+// one pass of 35 us at SCALE 23, whose counters are read with those of the
+// edge pass, where six with a readback after each take 130 us of kernels and
+// as much waiting.  An entry is looked at only if its index is in range.
 // kMap: with CoreBFS, the depth map (build_bfs_depth_map) is written to map
 // in the same pass instead of a check of the depths: entries of unknown depth
 // take that of the first ancestor with a known one, plus the steps.  map may

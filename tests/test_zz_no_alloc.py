@@ -3,10 +3,10 @@ allocate device memory (programs whose caching allocator owns the device,
 hosts with a fixed memory budget).  Its scratch lives in a fixed device array
 inside the library, so the test hands it only device inputs and outputs and
 checks its results against the engine's own b200bfs_run on the same graph,
-on two calls in a row.  It synchronises its stream once per level, so a
-stream being captured into a CUDA graph is refused before anything is
-enqueued, and the capture stays usable.  This file sorts last so that a run
-stopping at the first failure has already run every other test."""
+on two calls in a row.  It synchronises its stream, so a stream being captured
+into a CUDA graph is refused before anything is enqueued, and the capture
+stays usable.  This file sorts last so that a run stopping at the first
+failure has already run every other test."""
 import numpy as np
 import pytest
 
