@@ -58,9 +58,11 @@ struct Engine {
   // Freed memory that a build may keep for its later steps, and an engine
   // between its calls.  Other users of the device (a framework's allocator)
   // cannot take it back, so both are small beside the device's 180 GB, and
-  // only graphs that are small beside it as well profit in full: up to SCALE
-  // 22 a build's transient buffers, up to SCALE 26 those of the calls.
-  static constexpr uint64_t kBuildKeep = uint64_t(2) << 30;
+  // graphs that are small beside it as well profit in full: up to SCALE 24 a
+  // build's buffers, up to SCALE 26 those of the calls.  Rebuilding a graph
+  // with CoreBFS (ms, 2 GiB / 8 GiB / no limit): SCALE 22 33 / 33 / 33, SCALE
+  // 24 127 / 117 / 115, SCALE 26 - / 542 / 513.
+  static constexpr uint64_t kBuildKeep = uint64_t(8) << 30;
   static constexpr uint64_t kCallKeep = (uint64_t(1) << 30) + (1u << 20);
 
   // Keeps room for the transient buffers of the calls between searches (the

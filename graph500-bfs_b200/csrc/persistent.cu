@@ -395,10 +395,11 @@ bool run_bfs_core_persistent(const Graph& g, BfsState& st, cudaStream_t s, int s
   a.b2t = b2t_limit(st.R, edgefactor, beta);
   a.force_direction = opt.force_direction;
   a.seq = ++st.out_seq;
-  // Up to 80 K rows: one cluster of 16 blocks, whose barrier is the hardware's
-  // (us per search, cooperative grid / cluster: SCALE 12 62.3 / 60.1, SCALE 14
-  // 67.7 / 64.5, SCALE 16 77.5 / 69.8, its 2-core 76.1 / 68.5; SCALE 18, 170 K
-  // rows, 86.5 / 95.8: 16 SMs no longer do).
+  // Up to 80 K rows: one cluster of 16 blocks, whose barrier is the hardware's;
+  // beyond, 16 SMs no longer do.  us per search by rows, cooperative grid /
+  // cluster: 3 K 62.3 / 60.1, 47 K 77.2 / 76.5, 57 K 82.0 / 78.2, 64 K 92.4 /
+  // 86.0, 73 K (a 2-core) 77.2 / 79.5, 78 K 85.3 / 83.3, 90 K 88.0 / 85.4, 101 K
+  // 83.5 / 80.9, 123 K 92.9 / 96.3, 149 K 84.6 / 97.8, 174 K 92.3 / 101.9.
   // Else a cooperative grid.  Threads per SM: 1024 with the registers the level
   // code asks for (no spills) while a level is a few rounds of loads per warp;
   // from 6 M rows 2048 threads at 32 registers, whose loads in flight are worth

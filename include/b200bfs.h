@@ -63,7 +63,7 @@ enum {
 typedef struct b200bfs_handle b200bfs_handle;
 
 /* Without a budget an engine keeps device memory that it has freed for its next
- * allocations: up to 2 GiB while it builds a graph, and between calls up to 16
+ * allocations: up to 8 GiB while it builds a graph, and between calls up to 16
  * bytes per vertex id, at most 1 GiB (not counted in device_bytes).  Another
  * engine's allocation takes it back; b200bfs_end gives it back.  With a budget
  * nothing is kept. */
