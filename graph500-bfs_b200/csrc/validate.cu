@@ -51,7 +51,7 @@ __device__ __forceinline__ void max_up(unsigned long long* to, unsigned long lon
 // Value ranges, self-parents, depths and the highest used vertex
 // (find_max_used_vertex, benchmark_helper.hpp:564-582: rank or tree parent as
 // in has_edge) of every id, whichever of them the verdict turns out to need:
-// one pass of 35 us at SCALE 23, whose counters are read with those of the
+// one pass of 75 us at SCALE 23, whose counters are read with those of the
 // edge pass, where six with a readback after each take 130 us of kernels and
 // as much waiting.  An entry is looked at only if its index is in range.
 // kMap: with CoreBFS, the depth map (build_bfs_depth_map) is written to map
