@@ -86,16 +86,22 @@ __global__ void rank_kernel(const int32_t* __restrict__ inv, const uint32_t* __r
 
 // Places every edge in its source row; the stored value is the neighbour's
 // sort key nkey[v] (its row id, or its global degree rank when rows follow
-// the group order).
+// the group order).  *bad is set if a neighbour has no row: a list said to be
+// symmetric in which it is no edge's source.
 __global__ void scatter_kernel(const uint2* __restrict__ e, int64_t m, bool mirror,
                                const int32_t* __restrict__ rank, const int32_t* __restrict__ nkey,
                                const int64_t* __restrict__ raw_ptr,
-                               uint32_t* __restrict__ cursor, int32_t* __restrict__ raw) {
+                               uint32_t* __restrict__ cursor, int32_t* __restrict__ raw,
+                               unsigned long long* __restrict__ bad) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m;
        i += (int64_t)gridDim.x * blockDim.x) {
     uint2 x = e[i];
     if (x.x == x.y) continue;
     int32_t ra = rank[x.x], rb = rank[x.y];
+    if (rb < 0) {
+      *bad = 1;
+      continue;
+    }
     raw[raw_ptr[ra] + atomicAdd(cursor + ra, 1u)] = nkey[x.y];
     if (mirror) raw[raw_ptr[rb] + atomicAdd(cursor + rb, 1u)] = nkey[x.x];
   }
@@ -532,7 +538,14 @@ void build_csr(DeviceArena& arena, cudaStream_t s, const uint2* edges, int64_t m
   int32_t* raw = arena_alloc<int32_t>(arena, total, "raw adjacency");
   uint32_t* cursor = arena_alloc<uint32_t>(arena, R, "cursor");
   check_cuda(cudaMemsetAsync(cursor, 0, R * 4, s), "memset");
-  scatter_kernel<<<grid(m), B, 0, s>>>(edges, m, mirror, c.rank, nkey, raw_ptr, cursor, raw);
+  scatter_kernel<<<grid(m), B, 0, s>>>(edges, m, mirror, c.rank, nkey, raw_ptr, cursor, raw,
+                                       d_u64 + 1);
+  if (!mirror) {
+    unsigned long long bad = 0;
+    check_cuda(cudaMemcpyAsync(&bad, d_u64 + 1, 8, cudaMemcpyDeviceToHost, s), "copy");
+    check_cuda(cudaStreamSynchronize(s), "placement");
+    if (bad) throw Error{B200BFS_ERR_INVALID, "edge list is not symmetric"};
+  }
   if (nkey != c.rank) arena.free(nkey);
   arena.free(cursor);
 

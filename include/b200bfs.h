@@ -56,7 +56,8 @@ enum {
   /* The edge list given is already symmetric (each undirected edge present
    * in both directions, as the sym_edge_list passed to BfsBase::construct);
    * without this flag every edge is mirrored, as make_symmetry_edge_list
-   * (benchmark_helper.hpp:383-497) does. */
+   * (benchmark_helper.hpp:383-497) does.  A list with a vertex that edges lead
+   * to and none from is refused (B200BFS_ERR_INVALID). */
   B200BFS_BUILD_INPUT_SYMMETRIC = 1 << 2
 };
 

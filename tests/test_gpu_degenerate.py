@@ -92,3 +92,25 @@ def test_small_ragged_graphs_match_oracle(built, name, force):
             assert (derr, dcnt) == (err, cnt), (name, r)
     finally:
         e.close()
+
+
+@pytest.mark.parametrize("flags", [0, 2, 3])
+@pytest.mark.parametrize("hub", [3, 20000])
+def test_list_wrongly_said_to_be_symmetric(built, flags, hub):
+    """A neighbour that is no edge's source has no row: refused, also from a
+    row long enough to be sorted by bitmap, and the engine stays usable."""
+    import b200bfs
+
+    flags |= b200bfs.BUILD_INPUT_SYMMETRIC
+    i = np.arange(1, hub + 1)
+    half = np.stack([np.zeros(hub, int), i], 1).astype(np.int64)
+    both = np.concatenate([half, half[:, ::-1], [[1, 2], [2, 1]]])
+    engine = b200bfs.Engine(0)
+    with pytest.raises(b200bfs.B200BfsError) as ei:
+        engine.build_from_edges(np.concatenate([both, [[0, hub + 1]]]), flags=flags)
+    assert ei.value.code == 1
+    engine.build_from_edges(both, flags=flags)
+    engine.prepare(16)
+    engine.run(0)
+    assert engine.get_levels()[:hub + 1].tolist() == [0] + [1] * hub
+    engine.close()
